@@ -743,34 +743,31 @@ __device__ __forceinline__ void nee_surface(const Scene& S, Pool& P, Counters* c
     for (int li = 0; li < S.light_count; ++li) {
         const int le_i = S.light_entity[li];
         const float u0 = rng.u(), u1 = rng.u(), u2 = rng.u();
+        Vec3 lpos, rad;
+        float lpdf;
         if (le_i < 0) {
-            float lpdf;
             const Vec3 dir = env_sample(S, u0, u1, u2, &lpdf);
-            const Vec3 rad = env_radiance(S, dir);
+            rad = env_radiance(S, dir);
             if (black(rad)) continue;
-            const Vec3 lpos = env_emit_pos(S, sv.pos, dir);
-            const Vec3 to_light = normalize(lpos - sv.pos);
-            const Vec3 bf = bsdf_eval(bv, to_light, sv.wr);
-            if (black(bf)) continue;
-            const Vec3 contrib = coef * rad * bf *
-                                 (fabsf(cosv(to_light, sv.geo.z)) / (lpdf + side_pdf(to_light, bsdf_pdf(bv, to_light, sv.wr))));
-            push_shadow(P, c, sv.pos, to_light, eps, length(sv.pos - lpos) - eps, contrib, slot);
+            lpos = env_emit_pos(S, sv.pos, dir);
         } else {
-            const Entity& le = S.entities[le_i];
             LightSample ls;
-            if (!area_light_sample(S, le, sv.pos, u0, u1, u2, &ls)) continue;
+            if (!area_light_sample(S, S.entities[le_i], sv.pos, u0, u1, u2, &ls)) continue;
             if (black(ls.rad) || ls.pdf == 0.0f) continue;
-            const float slen = length(ls.pos - sv.pos) - eps;
-            if (slen <= eps) continue;
-            const Vec3 to_light = normalize(ls.pos - sv.pos);
-            const Vec3 bf = bsdf_eval(bv, to_light, sv.wr);
-            if (black(bf)) continue;
-            Vec3 tr(1.0f);
-            if (S.has_media) tr = medium_tr(S, medium_of(sv, e, to_light), ls.pos, sv.pos, rng, wd);
-            const Vec3 contrib = coef * tr * ls.rad * bf *
-                                 (fabsf(cosv(to_light, sv.geo.z)) / (ls.pdf + side_pdf(to_light, bsdf_pdf(bv, to_light, sv.wr))));
-            push_shadow(P, c, sv.pos, to_light, eps, slen, contrib, slot);
+            lpos = ls.pos;
+            rad = ls.rad;
+            lpdf = ls.pdf;
         }
+        const float slen = length(lpos - sv.pos) - eps;
+        if (le_i >= 0 && slen <= eps) continue;
+        const Vec3 to_light = normalize(lpos - sv.pos);
+        const BSDFValue bv_l = bsdf_eval_pdf(bv, to_light, sv.wr);
+        if (black(bv_l.f)) continue;
+        Vec3 tr(1.0f);
+        if (S.has_media && le_i >= 0) tr = medium_tr(S, medium_of(sv, e, to_light), lpos, sv.pos, rng, wd);
+        const Vec3 contrib = coef * tr * rad * bv_l.f *
+                             (fabsf(cosv(to_light, sv.geo.z)) / (lpdf + side_pdf(to_light, bv_l.pdf)));
+        push_shadow(P, c, sv.pos, to_light, eps, slen, contrib, slot);
     }
 }
 
@@ -1089,8 +1086,9 @@ __global__ void __launch_bounds__(128, ATRC_SHADE_MIN_BLOCKS) k_shade(Scene S, P
                     if (rng.u() < mix.c) {
                         const float g0 = rng.u(), g1 = rng.u(), g2 = rng.u();
                         bs.dir = guide_sample(mix, g0, g1, g2);
-                        bs.f = bsdf_eval(b, bs.dir, s.wr);
-                        pdf_bsdf = bsdf_pdf(b, bs.dir, s.wr);
+                        const BSDFValue v = bsdf_eval_pdf(b, bs.dir, s.wr);
+                        bs.f = v.f;
+                        pdf_bsdf = v.pdf;
                     } else {
                         const float u0 = rng.u(), u1 = rng.u(), u2 = rng.u();
                         bs = bsdf_sample(b, s.wr, u0, u1, u2);
