@@ -252,28 +252,54 @@ __device__ __forceinline__ bool disk_test(const RayState& r, float radius, float
     return true;
 }
 
-// Slab test of the four children of a wide node (seven 128-bit loads):
-// t[k] = entry distance of child k, +inf when it is missed or the slot is
-// empty.  Boxes are widened by 1.0000005 as in the binary test, so a box
-// that touches the ray in exact arithmetic is never culled.
+// min / max of three (one instruction on sm_100).
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// The bounds of a node's four children along one axis: lo[4], hi[4], one
+// 256-bit load (the node array never changes during a kernel).
+struct Bounds4 {
+    float lo[4], hi[4];
+};
+__device__ __forceinline__ Bounds4 ld_bounds(const float* p) {
+    Bounds4 b;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(b.lo[0]), "=f"(b.lo[1]), "=f"(b.lo[2]), "=f"(b.lo[3]), "=f"(b.hi[0]), "=f"(b.hi[1]), "=f"(b.hi[2]),
+          "=f"(b.hi[3])
+        : "l"(p));
+    return b;
+}
+
+// A box whose entry distance exceeds the current end of the ray by more than
+// this is not visited: the slack keeps a box that touches the ray in exact
+// arithmetic.
+__device__ __forceinline__ float box_reach(float t) { return t * 1.0000005f + 1e-30f; }
+
+// Slab test of the four children of a wide node (three 256-bit loads and one
+// of 128 bits): t[k] = entry distance of child k, +inf when it is missed or
+// the slot is empty.
 __device__ __forceinline__ void box4(const Bvh4Node* node, const RayState& r, float* t, int32_t* l) {
-    const float4* p = reinterpret_cast<const float4*>(node);
-    const float4 lx = __ldg(p), hx = __ldg(p + 1), ly = __ldg(p + 2), hy = __ldg(p + 3);
-    const float4 lz = __ldg(p + 4), hz = __ldg(p + 5);
-    const int4 lk = __ldg(reinterpret_cast<const int4*>(p + 6));
+    const float* p = reinterpret_cast<const float*>(node);
+    const Bounds4 x = ld_bounds(p), y = ld_bounds(p + 8), z = ld_bounds(p + 16);
+    const int4 lk = __ldg(reinterpret_cast<const int4*>(p + 24));
     const float ox = r.o.x * r.inv.x, oy = r.o.y * r.inv.y, oz = r.o.z * r.inv.z;
-    const float alx[4] = {lx.x, lx.y, lx.z, lx.w}, ahx[4] = {hx.x, hx.y, hx.z, hx.w};
-    const float aly[4] = {ly.x, ly.y, ly.z, ly.w}, ahy[4] = {hy.x, hy.y, hy.z, hy.w};
-    const float alz[4] = {lz.x, lz.y, lz.z, lz.w}, ahz[4] = {hz.x, hz.y, hz.z, hz.w};
     const int32_t al[4] = {lk.x, lk.y, lk.z, lk.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float a0 = fmaf(alx[k], r.inv.x, -ox), b0 = fmaf(ahx[k], r.inv.x, -ox);
-        const float a1 = fmaf(aly[k], r.inv.y, -oy), b1 = fmaf(ahy[k], r.inv.y, -oy);
-        const float a2 = fmaf(alz[k], r.inv.z, -oz), b2 = fmaf(ahz[k], r.inv.z, -oz);
-        const float lo = fmaxf(fmaxf(fminf(a0, b0), fminf(a1, b1)), fmaxf(fminf(a2, b2), r.tmin));
-        const float hi = fminf(fminf(fmaxf(a0, b0), fmaxf(a1, b1)), fminf(fmaxf(a2, b2), r.tmax));
-        const bool hit = al[k] != kEmptyLink && lo <= hi * 1.0000005f + 1e-30f;
+        const float a0 = fmaf(x.lo[k], r.inv.x, -ox), b0 = fmaf(x.hi[k], r.inv.x, -ox);
+        const float a1 = fmaf(y.lo[k], r.inv.y, -oy), b1 = fmaf(y.hi[k], r.inv.y, -oy);
+        const float a2 = fmaf(z.lo[k], r.inv.z, -oz), b2 = fmaf(z.hi[k], r.inv.z, -oz);
+        const float lo = fmaxf(max3(fminf(a0, b0), fminf(a1, b1), fminf(a2, b2)), r.tmin);
+        const float hi = fminf(min3(fmaxf(a0, b0), fmaxf(a1, b1), fmaxf(a2, b2)), r.tmax);
+        const bool hit = al[k] != kEmptyLink && lo <= box_reach(hi);
         t[k] = hit ? lo : INFINITY;
         l[k] = al[k];
     }
@@ -322,7 +348,15 @@ struct TraceCount {
 // traversal on GPUs", 2009): a thread that reaches a leaf while descending
 // parks it and keeps descending; the warp switches to leaf processing only
 // once every active lane holds a leaf, so node and leaf code run with most
-// lanes converged.  Top-level leaves (entities) switch the ray into the
+// lanes converged.  It also switches once fewer than 1 / kNodeShare of the
+// lanes that began the round still descend: the others would wait for the
+// longest descent of the warp (9 of 32 lanes were active on secondary rays).
+// Occlusion rays visit one leaf more per round, closest-hit rays every leaf
+// they meet.  Measured, 1/2 for closest hits and 1/3 with one leaf for
+// occlusion: 4M incoherent queries 1.99 -> 1.78 ms, the instanced frame's
+// traversal 20.08 -> 19.66 and its occlusion rays 7.72 -> 7.01 ms, the
+// occlusion rays of ao 2.41 -> 2.21 ms; 1/4 gave back half of it.
+// Top-level leaves (entities) switch the ray into the
 // entity's space and push a sentinel that restores the world ray when the
 // bottom-level tree is exhausted.  A ray whose stack would overflow or
 // whose visits exceed kMaxTraversalSteps ends with the watchdog set.
@@ -343,6 +377,7 @@ struct Tracer {
     int32_t best_e, best_tri, cur_entity, link, held;
     int steps;
     bool overflow, found;
+    static constexpr int kNodeShare = ANY ? 3 : 2;
 
     __device__ __forceinline__ void init(const Scene& S, int32_t* stk, Vec3 o, Vec3 d, float tmin, float tmax) {
         stack = stk;
@@ -455,6 +490,7 @@ struct Tracer {
     // lane holds a leaf, then the leaves.  Returns true when the ray is done.
     __device__ __forceinline__ bool step(const Scene& S, int* watchdog, TraceCount* cnt) {
         if (link == kDone && held == 0) return true;
+        const int n0 = __popc(__activemask());
         while (link >= 0) {
             if (++steps > kMaxTraversalSteps) { overflow = true; break; }
             if (COUNT) cnt->nodes++;
@@ -489,7 +525,8 @@ struct Tracer {
                 link = pop();
             }
             if (overflow) break;
-            if (!__any_sync(__activemask(), held == 0)) break;
+            const unsigned act = __activemask();
+            if (!__any_sync(act, held == 0) || __popc(act) * kNodeShare < n0) break;
         }
         if (overflow) { *watchdog = 1; return true; }
         // leaves: the parked one first, then any leaf / sentinel in `link`
@@ -510,7 +547,7 @@ struct Tracer {
             }
             const int32_t next = pop();
             link = visit_leaf(S, link, next, cnt);
-            if (found) break;
+            if (found || ANY) break;
         }
         if (overflow) { *watchdog = 1; return true; }
         return found || link == kDone;
