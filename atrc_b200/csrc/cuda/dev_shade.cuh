@@ -1116,7 +1116,7 @@ __device__ __forceinline__ Vec3 env_radiance(const Scene& S, Vec3 d) {
     return tex2d_lookup<false>(S, env.tex, u, v, Vec3(), false);
 }
 
-__device__ float env_pdf(const Scene& S, Vec3 d) {
+__device__ __forceinline__ float env_pdf(const Scene& S, Vec3 d) {
     const Env& env = S.env;
     if (env.type == ATRC_ENV_NATIVE_SKY) return 1 / (4 * kPi);
     const Vec3 dir = normalize(d);

@@ -74,6 +74,12 @@ __device__ __forceinline__ int warp_append(int* counter, bool pred) {
     return base + __popc(mask & ((1u << lane) - 1u));
 }
 
+// Warp sum of v added to *counter.
+__device__ __forceinline__ void warp_add(int* counter, int v) {
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && v > 0) atomicAdd(counter, v);
+}
+
 // ------------------------------------------------------------ ray queries
 // Persistent warps step their traversals round by round and refill the
 // lanes whose rays are done from `cursor`, as k_extend_fetch does: a batch of
@@ -147,7 +153,7 @@ enum PathFlags : int {
 
 struct Counters {
     int in, out;              // queue buffers read / written this iteration
-    int n_ext, n_next;        // paths to shade (continuations, then new camera hits) / continuations written
+    int n_ext, n_next;        // hits to shade / continuations written
     int n_shadow, n_finish;
     int n_guide;              // guide queries this iteration
     int n_sss;                // subsurface walks queued this iteration
@@ -156,7 +162,8 @@ struct Counters {
     int n_free, n_new, n_cont;  // free slots, samples that may be issued, continuations
     int gen_ticket;           // k_extend: samples taken this iteration (may run past n_new)
     int slot_ticket;          // k_extend: entries of the free-slot list reserved
-    int n_retired;            // k_extend: camera rays that met nothing and ended in place
+    int n_retired;            // k_extend: paths whose ray met nothing, ended in place
+    int n_taken, n_freed;     // k_extend: slots taken by camera hits, freed by ended continuations
     int free_ticket;          // k_free_slots: free slots listed
     int ext_ticket;           // k_free_slots: extend-queue entries written (slot order)
     unsigned long long gen_base, issued, total, completed;
@@ -292,8 +299,9 @@ struct Pool {
     float4* gb_albedo;            // albedo.xyz, denoise (renders with a G-buffer)
     float4* gb_normal;            // normal.xyz
     int* q[2];                    // extend queues
-    int* q_sorted;                // the extend queue sorted by material key
-    int* keys;                    // material key per extend-queue entry
+    int* q_hit;                   // paths whose ray met something, for k_shade
+    int* q_sorted;                // q_hit sorted by material key
+    int* keys;                    // material key per q_hit entry
     int* key_count;               // per key: entries this iteration
     int* key_cursor;              // per key: next write position in q_sorted
     int* q_finish;
@@ -349,11 +357,11 @@ constexpr int kIssuePools = 4;
 __global__ void k_begin(Counters* c, int cap) {
     c->iterations++;
     c->rays_shadow += c->n_shadow;
-    // what the last iteration issued, and the slots that its camera hits took
-    const int issued = min(c->gen_ticket, c->n_new), taken = c->n_ext - c->n_cont;
+    // what the last iteration issued, and the slots it took and freed
+    const int issued = min(c->gen_ticket, c->n_new);
     c->issued += issued;
     c->rays_closest += (unsigned long long)(c->n_cont + issued);
-    c->n_free += c->n_finish - taken;
+    c->n_free += c->n_finish + c->n_freed - c->n_taken;
     c->completed += c->n_finish + c->n_retired;
     const int n_cont = c->n_next;
     c->in = c->out;
@@ -365,10 +373,12 @@ __global__ void k_begin(Counters* c, int cap) {
     c->gen_ticket = 0;
     c->slot_ticket = 0;
     c->n_retired = 0;
+    c->n_taken = 0;
+    c->n_freed = 0;
     c->free_ticket = 0;
     c->ext_ticket = 0;
     c->n_cont = n_cont;
-    c->n_ext = n_cont;
+    c->n_ext = 0;
     c->n_next = 0;
     c->n_shadow = 0;
     c->n_finish = 0;
@@ -718,7 +728,7 @@ constexpr int kScatterKeys = 1024, kScatterPer = 8;
 
 __global__ void k_sort_scatter(Pool P, Counters* c, int nkeys) {
     __shared__ int run[kScatterKeys];
-    const int n = c->n_ext, in = c->in, lane = threadIdx.x & 31;
+    const int n = c->n_ext, lane = threadIdx.x & 31;
     if (nkeys > kScatterKeys) {
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
             const int key = P.keys[i];
@@ -727,7 +737,7 @@ __global__ void k_sort_scatter(Pool P, Counters* c, int nkeys) {
             int base = 0;
             if (lane == leader) base = atomicAdd(P.key_cursor + key, __popc(same));
             base = __shfl_sync(same, base, leader);
-            P.q_sorted[base + __popc(same & ((1u << lane) - 1u))] = P.q[in][i];
+            P.q_sorted[base + __popc(same & ((1u << lane) - 1u))] = P.q_hit[i];
         }
         return;
     }
@@ -740,7 +750,7 @@ __global__ void k_sort_scatter(Pool P, Counters* c, int nkeys) {
         for (int e = 0; e < kScatterPer; ++e) {
             const int i = i0 + e * int(blockDim.x) + int(threadIdx.x);
             key[e] = i < n ? P.keys[i] : -1;
-            slot[e] = i < n ? P.q[in][i] : 0;
+            slot[e] = i < n ? P.q_hit[i] : 0;
             const unsigned same = __match_any_sync(0xffffffffu, key[e]);
             const int leader = __ffs(same) - 1;
             int r = 0;
@@ -792,6 +802,30 @@ __global__ void __launch_bounds__(128) k_shsort_scatter(Pool P, Counters* c) {
     }
 }
 
+// A continuing path whose ray met nothing, as k_shade would end it: the
+// environment through the MIS term of its last vertex (direct_illum.cpp:130-192).
+__device__ __forceinline__ void retire_path(const Scene& S, const Params& p, Pool& P, int slot) {
+    const Rec8 mis = ld8(&P.sh[slot].mis), film = ld8(&P.sh[slot].film), ray = ld8(&P.tr[slot].ray);
+    const int flags = __float_as_int(mis.v[7]);
+    // the direction as stored: carried through the traversal in registers, its
+    // products were contracted differently from k_shade's
+    const Vec3 d = xyz2(ray);
+    Vec3 L = xyz(film);
+    if ((flags & PF_MIS) && S.env.type != ATRC_ENV_NONE) {
+        const Vec3 mis_f = xyz2(mis);
+        const float mis_pdf = mis.v[3];
+        const Vec3 le = env_radiance(S, d);
+        if (!black(le)) L += mis_f * le / ((flags & PF_MIS_DELTA) ? mis_pdf : mis_pdf + env_pdf(S, d));
+    }
+    const uint32_t vt = __float_as_uint(film.v[5]);
+    const int vi = int(vt >> kTileBits);
+    count_view(p, vi);
+    const float4 zero = make_float4(0, 0, 0, 0);
+    splat(p.views[vi], int(vt & ((1u << kTileBits) - 1u)), film.v[6], film.v[7], L, p.gbuffer ? P.gb_albedo[slot] : zero,
+          p.gbuffer ? P.gb_normal[slot] : zero);
+    P.slot_state[slot] = kSlotFree;
+}
+
 // Closest hits of one iteration: the continuing paths (unless CONT is off:
 // then k_extend_fetch traced them), then new camera samples.  Persistent
 // warps take 32 rays at a time from the counters, so no block waits for its
@@ -804,6 +838,10 @@ __global__ void __launch_bounds__(128) k_shsort_scatter(Pool P, Counters* c) {
 // splatted by four kernels; on the instanced workload, where the camera sees
 // the sky past most of its objects, four samples in five end here: 32 -> 20
 // iterations and 50.2 -> 39.5 ms per 16-spp step of 1920x1080.
+//
+// A continuation that meets nothing ends here too: k_shade reads hits only,
+// so its warps no longer hold lanes that only look up the sky (instanced step
+// 36.2 -> 33.3 ms, media 29.0 -> 25.9, subsurface Cornell 6.61 -> 6.36).
 template <int ISECT, bool COUNT, bool CONT>
 __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend(Scene S, Params p, Pool P, Counters* c) {
     constexpr int kMinLanes = 16;  // reserved slots a warp goes on with
@@ -812,7 +850,7 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend(S
     const int in = c->in, n_cont = c->n_cont, n_new = c->n_new, n_free = c->n_free;
     const unsigned long long gen = c->gen_base;
     TraceCount tc{0, 0, 0};
-    int wd = 0, retired = 0;
+    int wd = 0, retired = 0, freed = 0, taken = 0;
     bool cont = CONT && n_cont > 0;
     int a0 = 0, a1 = 0, b0 = 0, b1 = 0;  // reserved entries of the free-slot list
     for (;;) {
@@ -866,37 +904,47 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend(S
         h.tri = -1;
         bool hit = false;
         if (active) hit = trace_ray<ISECT, false, COUNT>(S, cs.o, cs.d, 0.0f, INFINITY, &h, &wd, &tc);
-        if (!old) {
-            if (active && !hit) {
+        if (active && !hit) {
+            if (!old) {
                 retire_miss(S, p, cs);
                 ++retired;
+            } else if (!p.gf.records) {
+                retire_path(S, p, P, slot);
+                ++retired;
+                ++freed;
             }
-            const unsigned hits = __ballot_sync(0xffffffffu, hit);
-            const int nh = __popc(hits);
-            if (nh == 0) continue;
-            int q0 = 0;
-            if (lane == 0) q0 = atomicAdd(&c->n_ext, nh);
-            q0 = __shfl_sync(0xffffffffu, q0, 0);
-            const int r = __popc(hits & below), from_a = min(nh, a1 - a0);
+        }
+        // recording renders end their paths in k_finish, which sets the
+        // records' targets: their misses go on to k_shade
+        const bool shade = hit || (old && active && p.gf.records);
+        const unsigned hits = __ballot_sync(0xffffffffu, shade);
+        const int nh = __popc(hits);
+        if (nh == 0) continue;
+        int q0 = 0;
+        if (lane == 0) q0 = atomicAdd(&c->n_ext, nh);
+        q0 = __shfl_sync(0xffffffffu, q0, 0);
+        const int r = __popc(hits & below);
+        if (!old) {
+            const int from_a = min(nh, a1 - a0);
             if (hit) {
                 slot = P.q_finish[r < from_a ? a0 + r : b0 + (r - from_a)];
-                i = q0 + r;
                 new_path(P, slot, cs, h, p.gbuffer);
-                P.q[in][i] = slot;
+                ++taken;
             }
             a0 += from_a;
             b0 += nh - from_a;
-            active = hit;
         }
-        if (active) {
+        if (shade) {
             if (old) store_hit(&P.tr[slot].hit, h, hit);
-            if (p.sort_mode != ATRC_SORT_NONE) count_key(S, P, p.sort_mode, p.nkeys, i, slot, hit, h.entity);
+            P.q_hit[q0 + r] = slot;
+            if (p.sort_mode != ATRC_SORT_NONE) count_key(S, P, p.sort_mode, p.nkeys, q0 + r, slot, hit, h.entity);
         }
         __syncwarp();
     }
     if (wd) atomicMax(&c->watchdog, wd);
-    for (int o = 16; o > 0; o >>= 1) retired += __shfl_down_sync(0xffffffffu, retired, o);
-    if (lane == 0 && retired > 0) atomicAdd(&c->n_retired, retired);
+    warp_add(&c->n_retired, retired);
+    warp_add(&c->n_freed, freed);
+    warp_add(&c->n_taken, taken);
     if (COUNT) flush_count(c->cnt_closest, tc);
 }
 
@@ -944,7 +992,9 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend_f
             h.t = h.u = h.v = 0.0f;
             const bool hit = tr.result(&h);
             store_hit(&P.tr[slot].hit, h, hit);
-            if (sort_mode != ATRC_SORT_NONE) count_key(S, P, sort_mode, nkeys, i, slot, hit, h.entity);
+            const int at = warp_append(&c->n_ext, true);
+            P.q_hit[at] = slot;
+            if (sort_mode != ATRC_SORT_NONE) count_key(S, P, sort_mode, nkeys, at, slot, hit, h.entity);
             i = -1;
         }
     }
@@ -1120,8 +1170,8 @@ __device__ __forceinline__ bool subsurface_sample(const Scene& S, const Material
 // serves are appended to a compact query list; gidx[i] is the query of
 // shade-queue entry i, or -1.
 __global__ void k_guide_features(Scene S, Params p, Pool P, Counters* c) {
-    const int n = c->n_ext, in = c->in;
-    const int* queue = p.sort_mode != ATRC_SORT_NONE ? P.q_sorted : P.q[in];
+    const int n = c->n_ext;
+    const int* queue = p.sort_mode != ATRC_SORT_NONE ? P.q_sorted : P.q_hit;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int slot = queue[i];
         GuideQuery q;
@@ -1154,9 +1204,9 @@ __global__ void k_guide_features(Scene S, Params p, Pool P, Counters* c) {
 }
 
 __global__ void __launch_bounds__(128, ATRC_SHADE_MIN_BLOCKS) k_shade(Scene S, Params p, Pool P, Counters* c) {
-    const int n = c->n_ext, in = c->in, out = c->out;
+    const int n = c->n_ext, out = c->out;
     const float eps = p.eps;
-    const int* queue = p.sort_mode != ATRC_SORT_NONE ? P.q_sorted : P.q[in];
+    const int* queue = p.sort_mode != ATRC_SORT_NONE ? P.q_sorted : P.q_hit;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int slot = queue[i];
         Trace2* const tp = P.tr + slot;
@@ -1817,7 +1867,7 @@ PoolLayout pool_layout(size_t cap, size_t shadow_cap, int nkeys) {
     take(11, cap * 4); take(12, cap * 4); take(13, cap * 4); take(14, cap * 4);
     take(15, shadow_cap * 16); take(16, shadow_cap * 16); take(17, shadow_cap * 16);
     take(18, cap * 4); take(19, cap * 4); take(20, size_t(nkeys) * 4); take(21, size_t(nkeys) * 4);
-    take(22, cap * 4);
+    take(22, cap * 4); take(27, cap * 4);
     take(23, shadow_cap * 4); take(24, shadow_cap * 4); take(25, kShadowKeys * 4); take(26, kShadowKeys * 4);
     L.total = (o + 255) & ~size_t(255);
     return L;
@@ -1842,6 +1892,7 @@ Pool pool_from(void* base, const PoolLayout& L, size_t cap, size_t shadow_cap) {
     P.key_count = reinterpret_cast<int*>(b + L.off[20]);
     P.key_cursor = reinterpret_cast<int*>(b + L.off[21]);
     P.q_sss = reinterpret_cast<int*>(b + L.off[22]);
+    P.q_hit = reinterpret_cast<int*>(b + L.off[27]);
     P.sh_key = reinterpret_cast<int*>(b + L.off[23]);
     P.sh_sorted = reinterpret_cast<int*>(b + L.off[24]);
     P.sh_count = reinterpret_cast<int*>(b + L.off[25]);

@@ -554,7 +554,7 @@ int atrc_cuda_stream_read_gbs(int device, uint64_t bytes, int passes, double* gb
  *  - The wavefront scratch (path pool, queues, shadow rays, counters) lives in
  *    a static device array of ATRC_NOALLOC_SCRATCH_BYTES that every GPU which
  *    loads this library keeps reserved until the process exits.  A path
- *    takes 188 bytes plus 56 per shadow ray it may emit in one iteration (one
+ *    takes 192 bytes plus 56 per shadow ray it may emit in one iteration (one
  *    per light for pt, ao_sample_count for ao), so the pool holds about 100k
  *    paths with one light.  Calls that leave room for fewer than 1024 paths
  *    (more than 434 lights, or ao_sample_count above 434) are rejected with
