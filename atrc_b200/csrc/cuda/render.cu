@@ -6,9 +6,8 @@
 // MIS direct lighting of src/tracer/src/render/direct_illum.cpp:11-278.
 //
 // Structure: a pool of P path slots in HBM (32-byte records); every
-// iteration runs six kernels over device-side queues, so the host never reads
+// iteration runs five kernels over device-side queues, so the host never reads
 // queue sizes inside the loop:
-//   begin     - 1 thread: flip queues, plan how many new camera samples to take
 //   free_slots- the free slots in ascending order
 //   extend    - closest hit of every continuing path, then camera rays
 //               (thin_lens.cpp:74-94) until the free slots hold their hits;
@@ -17,7 +16,8 @@
 //               medium sampling, emission, next-event estimation (one shadow
 //               ray per light), BSDF sampling
 //   shadow    - any hit for the shadow queue, unoccluded contributions added
-//   finish    - FP64 film splat of completed paths, slots returned
+//   finish    - FP64 film splat of completed paths, slots returned; its last
+//               block flips the queues and plans the next iteration's samples
 // The BSDF sample of a vertex serves both as the MIS-BSDF ray of
 // mis_sample_bsdf and as the continuation ray (the reference draws two
 // independent samples from the same distribution; the expectation of both
@@ -171,6 +171,10 @@ struct Counters {
     unsigned long long cnt_closest[3], cnt_shadow[3];  // nodes, tris, entities
     unsigned long long t_start;  // %globaltimer when the render's counters were reset
     int windows;                 // bounce-loop windows run by the device-side loop
+    // start of the iteration's stages (%globaltimer) and their device times so far
+    unsigned long long mark[4];      // traversal, shading, occlusion rays, film
+    unsigned long long stage_ns[3];
+    int finished_blocks;             // k_finish: blocks done this iteration
     int watchdog, done;
 };
 
@@ -182,6 +186,14 @@ __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
+}
+
+// The first thread of a stage's first kernel notes when it starts; the stage
+// ends where the next one starts.  (Event nodes in the captured loop did this
+// before: four more nodes per iteration, and not allowed in a loop that runs
+// on the device.)
+__device__ __forceinline__ void mark_stage(Counters* c, int stage) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) c->mark[stage] = global_ns();
 }
 
 __device__ __forceinline__ void flush_count(unsigned long long* dst, const TraceCount& tc) {
@@ -321,20 +333,6 @@ struct Pool {
 };
 constexpr int kShadowKeys = 4096;  // 16 x 16 x 16 origin cells
 
-__global__ void k_init(Pool P, int cap, int nkeys, Counters* c, unsigned long long total) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < cap) P.slot_state[i] = kSlotFree;
-    if (i < nkeys) P.key_count[i] = 0;
-    if (i < kShadowKeys) P.sh_count[i] = 0;
-    if (i == 0) {
-        memset(c, 0, sizeof(Counters));
-        c->n_free = cap;
-        c->total = total;
-        c->out = 0;
-        c->t_start = global_ns();
-    }
-}
-
 // End of one window of the device-side bounce loop: run another window
 // unless the work is done or a watchdog fired; after max_windows the loop
 // stops with kWatchdogLoop instead of running on (no path lives that long).
@@ -354,7 +352,12 @@ __global__ void k_loop_cond(Counters* c, cudaGraphConditionalHandle h, int max_w
 // host's progress and cancel polls (one per window of iterations) frequent.
 constexpr int kIssuePools = 4;
 
-__global__ void k_begin(Counters* c, int cap) {
+// Counters for the next iteration: what the last one did, how many samples
+// the next may issue, and whether the work is done.  Runs on one thread, at
+// the end of k_init and of k_finish's last block.
+__device__ void begin_iteration(Counters* c, int cap) {
+    if (c->iterations > 0)
+        for (int k = 0; k < 3; ++k) c->stage_ns[k] += c->mark[k + 1] - c->mark[k];
     c->iterations++;
     c->rays_shadow += c->n_shadow;
     // what the last iteration issued, and the slots it took and freed
@@ -387,6 +390,21 @@ __global__ void k_begin(Counters* c, int cap) {
     c->ext_cursor = 0;
     c->sh_cursor = 0;
     if (n_cont == 0 && c->n_new == 0) c->done = 1;
+}
+
+__global__ void k_init(Pool P, int cap, int nkeys, Counters* c, unsigned long long total) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < cap) P.slot_state[i] = kSlotFree;
+    if (i < nkeys) P.key_count[i] = 0;
+    if (i < kShadowKeys) P.sh_count[i] = 0;
+    if (i == 0) {
+        memset(c, 0, sizeof(Counters));
+        c->n_free = cap;
+        c->total = total;
+        c->out = 0;
+        c->t_start = global_ns();
+        begin_iteration(c, cap);
+    }
 }
 
 // Radiance and random stream of a path (20 of the film record's 32 bytes:
@@ -740,7 +758,10 @@ __device__ __forceinline__ void scan_counts(int* count, int* cursor, int nkeys) 
 
 __global__ void __launch_bounds__(1024) k_sort_scan(Pool P, int nkeys) { scan_counts(P.key_count, P.key_cursor, nkeys); }
 
-__global__ void __launch_bounds__(1024) k_shsort_scan(Pool P) { scan_counts(P.sh_count, P.sh_cursor, kShadowKeys); }
+__global__ void __launch_bounds__(1024) k_shsort_scan(Pool P, Counters* c) {
+    mark_stage(c, 2);
+    scan_counts(P.sh_count, P.sh_cursor, kShadowKeys);
+}
 
 // Scatter the extend queue into key order (order within a key is arbitrary).
 // A block takes kScatterPer x blockDim entries per pass, counts them per key
@@ -871,6 +892,7 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend(S
     constexpr int kMinLanes = 16;  // reserved slots a warp goes on with
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
+    if (CONT) mark_stage(c, 0);
     const int in = c->in, n_cont = c->n_cont, n_new = c->n_new, n_free = c->n_free;
     const unsigned long long gen = c->gen_base;
     TraceCount tc{0, 0, 0};
@@ -984,6 +1006,7 @@ constexpr int kRefillLanes = 16;
 template <int ISECT, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend_fetch(Scene S, Pool P, Counters* c,
                                                                                     int sort_mode, int nkeys) {
+    mark_stage(c, 0);
     const int n = c->n_cont, in = c->in;
     const int lane = threadIdx.x & 31;
     TraceCount tc{0, 0, 0};
@@ -1194,6 +1217,7 @@ __device__ __forceinline__ bool subsurface_sample(const Scene& S, const Material
 // serves are appended to a compact query list; gidx[i] is the query of
 // shade-queue entry i, or -1.
 __global__ void k_guide_features(Scene S, Params p, Pool P, Counters* c) {
+    mark_stage(c, 1);
     const int n = c->n_ext;
     const int* queue = p.sort_mode != ATRC_SORT_NONE ? P.q_sorted : P.q_hit;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1228,6 +1252,7 @@ __global__ void k_guide_features(Scene S, Params p, Pool P, Counters* c) {
 }
 
 __global__ void __launch_bounds__(128, ATRC_SHADE_MIN_BLOCKS) k_shade(Scene S, Params p, Pool P, Counters* c) {
+    if (!p.guide_on) mark_stage(c, 1);
     const int n = c->n_ext, out = c->out;
     const float eps = p.eps;
     const int* queue = p.sort_mode != ATRC_SORT_NONE ? P.q_sorted : P.q_hit;
@@ -1577,6 +1602,7 @@ __global__ void __launch_bounds__(128) k_subsurface(Scene S, Params p, Pool P, C
 
 template <int ISECT, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock, ATRC_SHADOW_MIN_BLOCKS) k_shadow(Scene S, Pool P, Counters* c) {
+    if (!P.shadow_sort) mark_stage(c, 2);
     const int n = min(c->n_shadow, P.shadow_cap);
     TraceCount tc{0, 0, 0};
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
@@ -1604,6 +1630,7 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_SHADOW_MIN_BLOCKS) k_shadow(
 // shadow queue.  Contributions and counts are those of k_shadow.
 template <int ISECT, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_shadow_fetch(Scene S, Pool P, Counters* c) {
+    if (!P.shadow_sort) mark_stage(c, 2);
     const int n = min(c->n_shadow, P.shadow_cap);
     const int lane = threadIdx.x & 31;
     TraceCount tc{0, 0, 0};
@@ -1644,7 +1671,10 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_shadow_f
     if (COUNT) flush_count(c->cnt_shadow, tc);
 }
 
+// Splats of the finished paths; the last block to end prepares the next
+// iteration (begin_iteration), which a kernel of one thread did before.
 __global__ void k_finish(Params p, Pool P, Counters* c) {
+    mark_stage(c, 3);
     const int n = c->n_finish;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int slot = P.q_finish[i];
@@ -1675,6 +1705,17 @@ __global__ void k_finish(Params p, Pool P, Counters* c) {
         splat(p.views[vi], tile, film.v[6], film.v[7], L, p.gbuffer ? P.gb_albedo[slot] : zero,
               p.gbuffer ? P.gb_normal[slot] : zero);
         P.slot_state[slot] = kSlotFree;
+    }
+    // the counters that begin_iteration resets are read above, before the
+    // block reports itself done
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&c->finished_blocks, 1) == int(gridDim.x) - 1) {
+            __threadfence();
+            c->finished_blocks = 0;
+            begin_iteration(c, P.cap);
+        }
     }
 }
 
@@ -1771,7 +1812,7 @@ struct DeviceSceneImpl {
     DevBuf pool_buf, counters, film_buf;
     // per-call resources kept between render calls
     static constexpr int kWindow = 4;  // wavefront iterations between host checks
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr, kev[kWindow * 4] = {};
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     static constexpr int kCopyChunks = 16;  // host-film download in pieces
     cudaEvent_t copy_ev[kCopyChunks] = {};
     void* pinned_counters = nullptr;
@@ -1787,7 +1828,11 @@ struct DeviceSceneImpl {
         view_stage_bytes = bytes;
     }
     cudaGraphExec_t window_exec = nullptr;  // the captured bounce-loop window
-    cudaGraphExec_t loop_exec = nullptr;    // the device-side bounce loop (batches)
+    cudaGraphExec_t loop_exec = nullptr;    // the device-side bounce loop
+    // everything the kept graphs' launches were captured with; a call with
+    // the same needs no capture (films, cameras and sample ranges are in the
+    // view table, which is not part of it)
+    std::vector<unsigned char> window_key, loop_key;
     void* stage = nullptr;             // pinned host staging for host films
     size_t stage_bytes = 0;
     // launch configuration (atrc_cuda_autotune chooses it; these are the
@@ -1814,7 +1859,6 @@ struct DeviceSceneImpl {
         if (!ev0) {
             CK(cudaEventCreate(&ev0));
             CK(cudaEventCreate(&ev1));
-            for (auto& e : kev) CK(cudaEventCreate(&e));
             for (auto& e : copy_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
         if (!pinned_counters) CK(cudaMallocHost(&pinned_counters, 512));
@@ -1830,7 +1874,6 @@ struct DeviceSceneImpl {
     ~DeviceSceneImpl() {
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
-        for (auto& e : kev) if (e) cudaEventDestroy(e);
         for (auto& e : copy_ev) if (e) cudaEventDestroy(e);
         if (window_exec) cudaGraphExecDestroy(window_exec);
         if (loop_exec) cudaGraphExecDestroy(loop_exec);
@@ -1917,7 +1960,7 @@ PoolLayout pool_layout(size_t cap, size_t shadow_cap, int nkeys) {
 
 Pool pool_from(void* base, const PoolLayout& L, size_t cap, size_t shadow_cap) {
     char* b = static_cast<char*>(base);
-    Pool P;
+    Pool P{};
     P.tr = reinterpret_cast<Trace2*>(b + L.off[0]);
     P.sh = reinterpret_cast<Shade2*>(b + L.off[1]);
     P.gb_albedo = reinterpret_cast<float4*>(b + L.off[7]);
@@ -2348,6 +2391,13 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
                        GuideImpl* guide = nullptr, bool record = false, double* view_seconds = nullptr,
                        bool device_loop = false) {
     const auto t_start = std::chrono::steady_clock::now();
+    // nobody to tell of progress and nobody to ask for a stop: the whole loop
+    // runs on the device.  With the stage times as device timestamps, the
+    // counters' turn inside k_finish and the graph kept between calls, an
+    // iteration is five nodes instead of ten: a 64 x 64 preview 1.60 -> 1.24 ms,
+    // the media's 52 short iterations 26.0 -> 24.4, the instanced step 32.4 ->
+    // 32.0
+    const bool use_loop = device_loop || (!should_stop && !progress);
     const AtrcRenderDesc* desc = descs;
     const AtrcFilm* film = films;
     DeviceSceneImpl& d = scene->impl;
@@ -2445,7 +2495,10 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
         d.ensure_view_stage(dbytes);
     }
     k_tiles<<<nviews, 32, 0, s>>>(p);
-    const int gsm = grid_for(d.sm_count, d.tuned_gen_blocks);
+    // k_free_slots and k_finish stride over the pool
+    auto scan_grid = [&](int threads) {
+        return int(std::min<size_t>(grid_for(d.sm_count, d.tuned_gen_blocks), (cap + threads - 1) / threads));
+    };
     // one path / ray per thread for the heavy kernels (grids cover the
     // pool; threads past the device-side count return at once)
     const int g_path = int((cap + 127) / 128), g_shadow = shadow_grid(shadow_cap, d.sm_count);
@@ -2454,9 +2507,7 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
     CK(cudaGetLastError());
     uint64_t launches = 2, ext_launches = 0;  // k_tiles, k_init
     cudaEvent_t ev0 = d.ev0, ev1 = d.ev1;
-    cudaEvent_t* kev = d.kev;
     const int window = DeviceSceneImpl::kWindow;
-    double t_ext = 0, t_shade = 0, t_shadow = 0;
     Counters hc{};
     static_assert(sizeof(Counters) <= 512, "pinned counter buffer too small");
     Counters* pinned = static_cast<Counters*>(d.pinned_counters);
@@ -2465,33 +2516,27 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
     // only; a watertight render ignores them
     const bool wt = desc->isect_mode == ATRC_ISECT_WATERTIGHT;
     const bool count = desc->count_traversal != 0 && !wt;
-    const int per_iter = 6 + (d.tuned_fetch ? 1 : 0) + (p.sort_mode != ATRC_SORT_NONE ? 2 : 0) + (guide ? 2 : 0) + (d.scene.has_subsurface ? 1 : 0) +
+    const int per_iter = 5 + (d.tuned_fetch ? 1 : 0) + (p.sort_mode != ATRC_SORT_NONE ? 2 : 0) + (guide ? 2 : 0) + (d.scene.has_subsurface ? 1 : 0) +
                          (P.shadow_sort ? 2 : 0);
     // The kernels of one window of `window` wavefront iterations.  The
     // kernels take their sizes from the device-side counters, so every window
-    // is the same sequence of launches.  `timed` records the events that
-    // split the window's device time into traversal, shading and shadow rays
-    // (event nodes are not allowed inside the device-side loop).
-    auto enqueue_window = [&](bool timed) {
+    // is the same sequence of launches.
+    auto enqueue_window = [&] {
         for (int k = 0; k < window; ++k) {
-            k_begin<<<1, 1, 0, s>>>(c, int(cap));
-            k_free_slots<<<gsm, d.tuned_gen_threads, 0, s>>>(p, P, c);
-            if (timed) CK(cudaEventRecordWithFlags(kev[k * 4 + 0], s, cudaEventRecordExternal));
+            k_free_slots<<<scan_grid(d.tuned_gen_threads), d.tuned_gen_threads, 0, s>>>(p, P, c);
             launch_extend(d, p, P, c, wt, count, s);
             if (p.sort_mode != ATRC_SORT_NONE) {
                 k_sort_scan<<<1, 1024, 0, s>>>(P, p.nkeys);
                 k_sort_scatter<<<d.sm_count * 8, 128, 0, s>>>(P, c, p.nkeys);
             }
-            if (timed) CK(cudaEventRecordWithFlags(kev[k * 4 + 1], s, cudaEventRecordExternal));
             if (guide) {
                 k_guide_features<<<g_path, 128, 0, s>>>(d.scene, p, P, c);
                 guide_infer(guide, &c->n_guide, s);
             }
             k_shade<<<g_path, 128, 0, s>>>(d.scene, p, P, c);
             if (d.scene.has_subsurface) k_subsurface<<<g_path, 128, 0, s>>>(d.scene, p, P, c);
-            if (timed) CK(cudaEventRecordWithFlags(kev[k * 4 + 2], s, cudaEventRecordExternal));
             if (P.shadow_sort) {
-                k_shsort_scan<<<1, 1024, 0, s>>>(P);
+                k_shsort_scan<<<1, 1024, 0, s>>>(P, c);
                 k_shsort_scatter<<<d.sm_count * 8, 128, 0, s>>>(P, c);
             }
             if (d.tuned_shadow_fetch) {
@@ -2506,13 +2551,27 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
             } else {
                 k_shadow<ISECT_FAST, false><<<g_shadow, 128, 0, s>>>(d.scene, P, c);
             }
-            if (timed) CK(cudaEventRecordWithFlags(kev[k * 4 + 3], s, cudaEventRecordExternal));
-            k_finish<<<gsm, d.tuned_fin_threads, 0, s>>>(p, P, c);
+            k_finish<<<scan_grid(d.tuned_fin_threads), d.tuned_fin_threads, 0, s>>>(p, P, c);
         }
         CK(cudaGetLastError());
     };
+    std::vector<unsigned char> key;
+    auto add_key = [&](const void* a, size_t bytes) {
+        key.insert(key.end(), static_cast<const unsigned char*>(a), static_cast<const unsigned char*>(a) + bytes);
+    };
+    {
+        const int ints[] = {int(cap), d.tuned_gen_blocks, d.tuned_gen_threads, d.tuned_fin_threads, d.tuned_fetch,
+                            d.tuned_shadow_fetch, int(wt), int(count), nviews};
+        add_key(&d.scene, sizeof(d.scene));
+        add_key(&p, sizeof(p));
+        add_key(&P, sizeof(P));
+        add_key(&c, sizeof(c));
+        add_key(ints, sizeof(ints));
+    }
+    // a guide's launches hold its own buffers and settings: captured anew
+    auto keep = [&](const std::vector<unsigned char>& k) { return !guide && k == key; };
     CK(cudaEventRecord(ev0, s));
-    if (device_loop) {
+    if (use_loop) {
         // The whole bounce loop is one graph launch: a WHILE conditional node
         // whose body is one window followed by k_loop_cond, which decides on
         // the device whether another window runs.  The host waits once, at
@@ -2526,37 +2585,42 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
             (unsigned long long)std::max(desc->max_depth, 1) + (unsigned long long)std::max(desc->specular_depth, 0) + 8;
         const unsigned long long bound_iters = 4ULL * (total / cap + 2) * per_path + 256;
         const int max_windows = int(std::min<unsigned long long>(bound_iters / window + 1, (1ULL << 30)));
-        cudaGraph_t outer = nullptr;
-        CK(cudaGraphCreate(&outer, 0));
-        struct GraphOwner {
-            cudaGraph_t g;
-            ~GraphOwner() { cudaGraphDestroy(g); }
-        } owner{outer};
-        cudaGraphConditionalHandle handle;
-        CK(cudaGraphConditionalHandleCreate(&handle, outer, 1, cudaGraphCondAssignDefault));
-        cudaGraphNodeParams np{};
-        np.type = cudaGraphNodeTypeConditional;
-        np.conditional.handle = handle;
-        np.conditional.type = cudaGraphCondTypeWhile;
-        np.conditional.size = 1;
-        cudaGraphNode_t node = nullptr;
-        CK(cudaGraphAddNode(&node, outer, nullptr, 0, &np));
-        {
-            BodyCapture body(s, np.conditional.phGraph_out[0]);
-            enqueue_window(false);
-            k_loop_cond<<<1, 1, 0, s>>>(c, handle, max_windows);
-            CK(cudaGetLastError());
-            body.end();
+        add_key(&max_windows, sizeof(max_windows));
+        if (!d.loop_exec || !keep(d.loop_key)) {
+            cudaGraph_t outer = nullptr;
+            CK(cudaGraphCreate(&outer, 0));
+            struct GraphOwner {
+                cudaGraph_t g;
+                ~GraphOwner() { cudaGraphDestroy(g); }
+            } owner{outer};
+            cudaGraphConditionalHandle handle;
+            CK(cudaGraphConditionalHandleCreate(&handle, outer, 1, cudaGraphCondAssignDefault));
+            cudaGraphNodeParams np{};
+            np.type = cudaGraphNodeTypeConditional;
+            np.conditional.handle = handle;
+            np.conditional.type = cudaGraphCondTypeWhile;
+            np.conditional.size = 1;
+            cudaGraphNode_t node = nullptr;
+            CK(cudaGraphAddNode(&node, outer, nullptr, 0, &np));
+            {
+                BodyCapture body(s, np.conditional.phGraph_out[0]);
+                enqueue_window();
+                k_loop_cond<<<1, 1, 0, s>>>(c, handle, max_windows);
+                CK(cudaGetLastError());
+                body.end();
+            }
+            d.loop_key.clear();
+            d.loop_exec = instantiate_or_update(d.loop_exec, outer);
+            if (!guide) d.loop_key = key;
         }
-        d.loop_exec = instantiate_or_update(d.loop_exec, outer);
         CK(cudaGraphLaunch(d.loop_exec, s));
         CK(cudaMemcpyAsync(pinned, c, sizeof(Counters), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(d.view_stage, p.view_time, dbytes, cudaMemcpyDeviceToHost, s));
+        if (dbytes) CK(cudaMemcpyAsync(d.view_stage, p.view_time, dbytes, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         hc = *pinned;
         launches += uint64_t(hc.windows) * (uint64_t(window) * per_iter + 1);
         ext_launches = uint64_t(hc.windows) * window;
-        if (view_seconds) {
+        if (view_seconds && dbytes) {
             const unsigned long long* vt = static_cast<const unsigned long long*>(d.view_stage);
             for (int v = 0; v < nviews; ++v)
                 view_seconds[v] = vt[v] >= hc.t_start ? double(vt[v] - hc.t_start) * 1e-9 : 0.0;
@@ -2569,13 +2633,15 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
         // polls progress and the cancel callback between windows.  The
         // executable graph is kept with the scene and updated in place when
         // the next call's parameters differ.
-        {
+        if (!d.window_exec || !keep(d.window_key)) {
+            d.window_key.clear();
             CaptureGuard capg(s);
-            enqueue_window(true);
+            enqueue_window();
             CK(cudaMemcpyAsync(pinned, c, sizeof(Counters), cudaMemcpyDeviceToHost, s));
             cudaGraph_t g = capg.end();
             d.window_exec = instantiate_or_update(d.window_exec, g);
             cudaGraphDestroy(g);
+            if (!guide) d.window_key = key;
         }
         for (;;) {
             CK(cudaGraphLaunch(d.window_exec, s));
@@ -2583,15 +2649,6 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
             ext_launches += window;
             CK(cudaStreamSynchronize(s));
             hc = *pinned;
-            for (int k = 0; k < window; ++k) {
-                float a = 0, b2 = 0, e3 = 0;
-                CK(cudaEventElapsedTime(&a, kev[k * 4 + 0], kev[k * 4 + 1]));
-                CK(cudaEventElapsedTime(&b2, kev[k * 4 + 1], kev[k * 4 + 2]));
-                CK(cudaEventElapsedTime(&e3, kev[k * 4 + 2], kev[k * 4 + 3]));
-                t_ext += a * 1e-3;
-                t_shade += b2 * 1e-3;
-                t_shadow += e3 * 1e-3;
-            }
             if (hc.watchdog) { status = ATRC_ERR_WATCHDOG; break; }
             if (hc.done) break;
             if (progress) progress(100.0 * double(hc.completed) / double(std::max(1ULL, total)), user);
@@ -2653,9 +2710,9 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
         stats->iterations = hc.iterations;
         stats->kernel_launches = launches;
         stats->watchdog_flags = uint64_t(hc.watchdog);
-        stats->extend_seconds = t_ext;
-        stats->shade_seconds = t_shade;
-        stats->shadow_seconds = t_shadow;
+        stats->extend_seconds = hc.stage_ns[0] * 1e-9;
+        stats->shade_seconds = hc.stage_ns[1] * 1e-9;
+        stats->shadow_seconds = hc.stage_ns[2] * 1e-9;
         stats->h2d_bytes = 0;
         stats->d2h_bytes = d2h;
         stats->extend_launches = ext_launches;
@@ -3007,7 +3064,9 @@ int atrc_cuda_render_noalloc(AtrcScene* scene, const AtrcRenderDesc* desc, const
         k_tiles<<<1, 32, 0, s>>>(p);
         Pool P = pool_from(base + counters_bytes + tiles_bytes, L, cap, shadow_cap);
         set_shadow_sort(&P, d.scene, d.tuned_shadow_sort);
-        const int gsm = grid_for(d.sm_count, d.tuned_gen_blocks);
+        auto scan_grid = [&](int threads) {
+            return int(std::min<size_t>(grid_for(d.sm_count, d.tuned_gen_blocks), (cap + threads - 1) / threads));
+        };
         const int g_path = int((cap + 127) / 128), g_shadow = shadow_grid(shadow_cap, d.sm_count);
         // k_init rewrites the counters and the slot states (all state that must
         // start from a known value)
@@ -3019,8 +3078,7 @@ int atrc_cuda_render_noalloc(AtrcScene* scene, const AtrcRenderDesc* desc, const
         const auto t0 = std::chrono::steady_clock::now();
         for (;;) {
             for (int k = 0; k < DeviceSceneImpl::kWindow; ++k) {
-                k_begin<<<1, 1, 0, s>>>(c, int(cap));
-                k_free_slots<<<gsm, d.tuned_gen_threads, 0, s>>>(p, P, c);
+                k_free_slots<<<scan_grid(d.tuned_gen_threads), d.tuned_gen_threads, 0, s>>>(p, P, c);
                 const int g_fetch = d.sm_count * ATRC_TRACE_MIN_BLOCKS;
                 launch_extend(d, p, P, c, wt, false, s);
                 if (p.sort_mode != ATRC_SORT_NONE) {
@@ -3034,7 +3092,7 @@ int atrc_cuda_render_noalloc(AtrcScene* scene, const AtrcRenderDesc* desc, const
                     launches += 1;
                 }
                 if (P.shadow_sort) {
-                    k_shsort_scan<<<1, 1024, 0, s>>>(P);
+                    k_shsort_scan<<<1, 1024, 0, s>>>(P, c);
                     k_shsort_scatter<<<d.sm_count * 8, 128, 0, s>>>(P, c);
                     launches += 2;
                 }
@@ -3046,8 +3104,8 @@ int atrc_cuda_render_noalloc(AtrcScene* scene, const AtrcRenderDesc* desc, const
                     k_shadow<ISECT_WATERTIGHT, false><<<g_shadow, 128, 0, s>>>(d.scene, P, c);
                 else
                     k_shadow<ISECT_FAST, false><<<g_shadow, 128, 0, s>>>(d.scene, P, c);
-                k_finish<<<gsm, d.tuned_fin_threads, 0, s>>>(p, P, c);
-                launches += 6 + (d.tuned_fetch ? 1 : 0);
+                k_finish<<<scan_grid(d.tuned_fin_threads), d.tuned_fin_threads, 0, s>>>(p, P, c);
+                launches += 5 + (d.tuned_fetch ? 1 : 0);
                 ext_launches += 1;
             }
             CK(cudaGetLastError());
