@@ -356,6 +356,7 @@ struct TraceCount {
 // occlusion: 4M incoherent queries 1.99 -> 1.78 ms, the instanced frame's
 // traversal 20.08 -> 19.66 and its occlusion rays 7.72 -> 7.01 ms, the
 // occlusion rays of ao 2.41 -> 2.21 ms; 1/4 gave back half of it.
+// EARLY = false leaves both out (kernels that refill finished lanes).
 // Top-level leaves (entities) switch the ray into the
 // entity's space and push a sentinel that restores the world ray when the
 // bottom-level tree is exhausted.  A ray whose stack would overflow or
@@ -363,7 +364,7 @@ struct TraceCount {
 // The traversal stack is the caller's local array (kStackSize entries, the
 // deeper ones past a shared-memory ring with ATRC_STACK_RING), kept out of
 // the struct so that the scalar state stays in registers.
-template <int ISECT, bool ANY, bool COUNT = false>
+template <int ISECT, bool ANY, bool COUNT = false, bool EARLY = true>
 struct Tracer {
 #if ATRC_STACK_RING > 0
     int32_t* ring;
@@ -490,7 +491,7 @@ struct Tracer {
     // lane holds a leaf, then the leaves.  Returns true when the ray is done.
     __device__ __forceinline__ bool step(const Scene& S, int* watchdog, TraceCount* cnt) {
         if (link == kDone && held == 0) return true;
-        const int n0 = __popc(__activemask());
+        const int n0 = EARLY ? __popc(__activemask()) : 0;
         while (link >= 0) {
             if (++steps > kMaxTraversalSteps) { overflow = true; break; }
             if (COUNT) cnt->nodes++;
@@ -526,7 +527,7 @@ struct Tracer {
             }
             if (overflow) break;
             const unsigned act = __activemask();
-            if (!__any_sync(act, held == 0) || __popc(act) * kNodeShare < n0) break;
+            if (!__any_sync(act, held == 0) || (EARLY && __popc(act) * kNodeShare < n0)) break;
         }
         if (overflow) { *watchdog = 1; return true; }
         // leaves: the parked one first, then any leaf / sentinel in `link`
@@ -547,7 +548,7 @@ struct Tracer {
             }
             const int32_t next = pop();
             link = visit_leaf(S, link, next, cnt);
-            if (found || ANY) break;
+            if (found || (ANY && EARLY)) break;
         }
         if (overflow) { *watchdog = 1; return true; }
         return found || link == kDone;

@@ -1011,7 +1011,7 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend_f
     const int lane = threadIdx.x & 31;
     TraceCount tc{0, 0, 0};
     int32_t stack[kStackSize];
-    Tracer<ISECT, false, COUNT> tr;
+    Tracer<ISECT, false, COUNT, false> tr;
     int i = -1, slot = -1, wd = 0;
     bool drained = false;
     for (;;) {
@@ -1624,7 +1624,9 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_SHADOW_MIN_BLOCKS) k_shadow(
     if (COUNT) flush_count(c->cnt_shadow, tc);
 }
 
-// k_shadow with dynamic ray fetch, as k_extend_fetch: persistent warps
+// k_shadow with dynamic ray fetch, as k_extend_fetch (with rounds that end
+// when every lane holds a leaf: a refill needs idle lanes, not early rounds,
+// whose test cost 1.3 of 8.5 ms here): persistent warps
 // step their any-hit traversals round by round and refill the lanes whose
 // rays are done (occluded at the first hit, or through the scene) from the
 // shadow queue.  Contributions and counts are those of k_shadow.
@@ -1635,7 +1637,7 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_shadow_f
     const int lane = threadIdx.x & 31;
     TraceCount tc{0, 0, 0};
     int32_t stack[kStackSize];
-    Tracer<ISECT, true, COUNT> tr;
+    Tracer<ISECT, true, COUNT, false> tr;
     int i = -1, wd = 0;
     bool drained = false;
     for (;;) {
@@ -1847,6 +1849,7 @@ struct DeviceSceneImpl {
     int tuned_queue = 0;          // extend queue in slot order (1) or shade order (0)
     int tuned_shadow_fetch = 0;   // k_shadow_fetch instead of k_shadow
     int tuned_shadow_sort = 0;    // shadow queue in origin-cell order
+    int default_sort = ATRC_SORT_NONE;  // tuned_sort until the scene is tuned
     int tuned_trials = 0;
     double tuned_ms = 0, default_ms = 0;
     DevBuf tune_film;
@@ -1854,6 +1857,22 @@ struct DeviceSceneImpl {
         p->sort_mode = requested == ATRC_SORT_AUTO ? tuned_sort : requested;
         p->slot_queue = tuned_queue;
         p->nkeys = std::max(scene.material_count, kMaterialTypes) + 2;
+    }
+    // The sort of a scene that was not tuned: by material type where shading
+    // differs most between neighbouring paths, media (tracking loops against
+    // surfaces; 767x511x8: 24.4 -> 22.9 ms) and Disney among other materials
+    // (subsurface Cornell 6.01 -> 5.01).  Where all is Disney the sort only
+    // costs (room 49.5 -> 50.5), and a box of Lambertian walls gains nothing
+    // (10.6 -> 10.8): black surfaces end their paths and do not count.
+    void choose_default_sort(const std::vector<Entity>& entities, const std::vector<Material>& materials) {
+        bool disney = false, other = false;
+        for (const Entity& e : entities) {
+            const int t = materials[e.material].type;
+            if (t == ATRC_MAT_DISNEY) disney = true;
+            else if (t != ATRC_MAT_IDEAL_BLACK) other = true;
+        }
+        default_sort = scene.has_media || (disney && other) ? ATRC_SORT_TYPE : ATRC_SORT_NONE;
+        tuned_sort = default_sort;
     }
     void ensure_render_resources() {
         if (!ev0) {
@@ -2173,6 +2192,7 @@ int atrc_cuda_scene_create(const AtrcSceneDesc* desc, AtrcScene** out) {
         S.env.alias_idx = upload(d.env_alias_idx, hs->env_alias_idx, s);
         S.eps = 3e-4f;
         d.scene = S;
+        d.choose_default_sort(hs->entities, hs->materials);
         d.watchdog.alloc(2 * sizeof(int));  // [0] watchdog code, [1] ray-query cursor
         // load the module's static scratch onto this device now, so that
         // atrc_cuda_render_noalloc neither allocates nor looks it up itself
@@ -2885,7 +2905,7 @@ int atrc_cuda_autotune(AtrcScene* scene, const AtrcRenderDesc* desc, int32_t tri
             return best;
         };
         // defaults first (one warm-up trial compiles nothing but pages in)
-        AtrcTuning base{1 << 21, ATRC_SORT_NONE, 16, 256, 128, 0, 0, 0, 0, 0};
+        AtrcTuning base{1 << 21, d.default_sort, 16, 256, 128, 0, 0, 0, 0, 0};
         if (!pool_fits(base.path_pool)) base.path_pool = 1 << 19;
         measure(base);
         const double base_ms = measure(base);
