@@ -515,9 +515,16 @@ struct Tracer {
                 if (tc[0] == INFINITY) {
                     link = pop();
                 } else {
-                    if (tc[3] != INFINITY) push(lc[3]);
-                    if (tc[2] != INFINITY) push(lc[2]);
-                    if (tc[1] != INFINITY) push(lc[1]);
+                    // sorted: a child is hit only if those before it are, and
+                    // mostly one or two are (three tests in a row instead:
+                    // the room's traversal 17.2 -> 17.6 ms)
+                    if (tc[1] != INFINITY) {
+                        if (tc[2] != INFINITY) {
+                            if (tc[3] != INFINITY) push(lc[3]);
+                            push(lc[2]);
+                        }
+                        push(lc[1]);
+                    }
                     link = lc[0];
                 }
             }
