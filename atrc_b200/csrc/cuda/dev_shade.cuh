@@ -227,23 +227,21 @@ struct BSDF {
     int type;
     Coord geo, shd;
     Vec3 albedo;
-    // disney
-    Vec3 C, Ctint, spec_scale;
-    float metallic, roughness, spec_tint, sheen, sheen_tint, clearcoat, transmission, IOR;
-    float trans_ax, trans_ay, ax, ay, cc_rough;
-    float w_diffuse, w_specular, w_clearcoat, w_transmission;
+    const DisneyParams* dp;  // disney: the material's, or those of this vertex
+    float roughness, ax, ay;  // metal
     float eps;
     bool disney_fixed;  // sample the diffuse lobe instead of falling through
     // mirror / metal: conductor Fresnel (eta_in / eta_out)^2, (k / eta_out)^2
     // and the colour it is multiplied with
     Vec3 eta2, etak2, rc;
-    // glass: ior (inside), reflection and refraction colours
+    // glass: ior (inside; of the medium for kMatSeparable), reflection and
+    // refraction colours
     float glass_ior;
     Vec3 refl_c, refr_c;
     // phong: diffuse and specular colours, exponent, component weights
     Vec3 pd, ps;
     float pns, wd, wsp;
-    // separable subsurface exit (kMatSeparable): eta in IOR, 1 - 2 FM1(1/eta)
+    // separable subsurface exit (kMatSeparable): eta in glass_ior, 1 - 2 FM1(1/eta)
     float sep_ci;
 };
 
@@ -391,7 +389,7 @@ __device__ __forceinline__ float phong_spec_pdf(const BSDF& b, Vec3 lwi, Vec3 lw
     return pow_cos_pdf(b.pns, normalize(l).z);
 }
 
-__device__ void disney_init(BSDF& b, Vec3 base, float met, float rough, float trans, float trans_rough, float ior,
+__device__ __forceinline__ void disney_init(DisneyParams& b, Vec3 base, float met, float rough, float trans, float trans_rough, float ior,
                             Vec3 spec_scale, float spec_tint, float aniso, float sheen, float sheen_tint, float cc,
                             float cc_gloss) {
     b.C = base;
@@ -419,41 +417,40 @@ __device__ void disney_init(BSDF& b, Vec3 base, float met, float rough, float tr
     b.w_transmission = A * trans;
     b.w_specular = B * 2 / (2 + cc);
     b.w_clearcoat = B * cc / (2 + cc);
-    b.albedo = base;
 }
 
 __device__ Vec3 disney_f_trans(const BSDF& b, Vec3 lwi, Vec3 lwo) {
     const float ci = lwi.z, co = lwo.z;
-    const float eta = co > 0 ? b.IOR : 1 / b.IOR;
+    const float eta = co > 0 ? b.dp->IOR : 1 / b.dp->IOR;
     Vec3 lwh = normalize(lwo + eta * lwi);
     if (lwh.z < 0) lwh = -lwh;
     const float cd = dot(lwo, lwh);
-    const float F = dielectric_fresnel(b.IOR, 1, cd);
+    const float F = dielectric_fresnel(b.dp->IOR, 1, cd);
     float sph, cph, spi, cpi, spo, cpo;
     sincos_phi(lwh, &sph, &cph);
     sincos_phi(lwi, &spi, &cpi);
     sincos_phi(lwo, &spo, &cpo);
-    const float D = aniso_gtr2(sph, cph, cos_2_sin(lwh.z), lwh.z, b.trans_ax, b.trans_ay);
-    const float G = smith_aniso_gtr2(cpi, spi, b.trans_ax, b.trans_ay, tan_theta(lwi)) *
-                    smith_aniso_gtr2(cpo, spo, b.trans_ax, b.trans_ay, tan_theta(lwo));
+    const float D = aniso_gtr2(sph, cph, cos_2_sin(lwh.z), lwh.z, b.dp->trans_ax, b.dp->trans_ay);
+    const float G = smith_aniso_gtr2(cpi, spi, b.dp->trans_ax, b.dp->trans_ay, tan_theta(lwi)) *
+                    smith_aniso_gtr2(cpo, spo, b.dp->trans_ax, b.dp->trans_ay, tan_theta(lwo));
     const float sdem = cd + eta * dot(lwi, lwh);
     const float corr = 1 / eta;
     const float val = (1 - F) * D * G * eta * eta * dot(lwi, lwh) * dot(lwo, lwh) * corr * corr / (ci * co * sdem * sdem);
-    const float tf = co > 0 ? b.transmission : 1.0f;
-    return (1 - b.metallic) * tf * Vec3(sqrtf(b.C.x), sqrtf(b.C.y), sqrtf(b.C.z)) * fabsf(val);
+    const float tf = co > 0 ? b.dp->transmission : 1.0f;
+    return (1 - b.dp->metallic) * tf * Vec3(sqrtf(b.dp->C.x), sqrtf(b.dp->C.y), sqrtf(b.dp->C.z)) * fabsf(val);
 }
 
 __device__ Vec3 disney_f_inner(const BSDF& b, Vec3 lwi, Vec3 lwo) {
     const Vec3 lwh = -normalize(lwi + lwo);
-    const float F = dielectric_fresnel(b.IOR, 1, dot(lwo, lwh));
+    const float F = dielectric_fresnel(b.dp->IOR, 1, dot(lwo, lwh));
     float sph, cph, spi, cpi, spo, cpo;
     sincos_phi(lwh, &sph, &cph);
     sincos_phi(lwi, &spi, &cpi);
     sincos_phi(lwo, &spo, &cpo);
-    const float D = aniso_gtr2(sph, cph, cos_2_sin(lwh.z), lwh.z, b.trans_ax, b.trans_ay);
-    const float G = smith_aniso_gtr2(cpi, spi, b.trans_ax, b.trans_ay, tan_theta(lwi)) *
-                    smith_aniso_gtr2(cpo, spo, b.trans_ax, b.trans_ay, tan_theta(lwo));
-    return b.transmission * b.C * fabsf(F * D * G / (4 * lwi.z * lwo.z));
+    const float D = aniso_gtr2(sph, cph, cos_2_sin(lwh.z), lwh.z, b.dp->trans_ax, b.dp->trans_ay);
+    const float G = smith_aniso_gtr2(cpi, spi, b.dp->trans_ax, b.dp->trans_ay, tan_theta(lwi)) *
+                    smith_aniso_gtr2(cpo, spo, b.dp->trans_ax, b.dp->trans_ay, tan_theta(lwo));
+    return b.dp->transmission * b.dp->C * fabsf(F * D * G / (4 * lwi.z * lwo.z));
 }
 
 __device__ __forceinline__ bool is_aggregate(int type) { return type == ATRC_MAT_METAL || type == ATRC_MAT_PHONG; }
@@ -461,12 +458,12 @@ __device__ __forceinline__ bool is_aggregate(int type) { return type == ATRC_MAT
 // SeparableBSDF::eval (separable.cpp:50-60): (1 - Fr(cos wi)) / (c pi) eta^2
 // for any wi, below the surface too
 __device__ __forceinline__ Vec3 separable_eval(const BSDF& b, Vec3 wi) {
-    const float fr = dielectric_fresnel(b.IOR, 1.0f, cosv(wi, b.geo.z));
-    return Vec3((1.0f - fr) / (b.sep_ci * kPi) * b.IOR * b.IOR);
+    const float fr = dielectric_fresnel(b.glass_ior, 1.0f, cosv(wi, b.geo.z));
+    return Vec3((1.0f - fr) / (b.sep_ci * kPi) * b.glass_ior * b.glass_ior);
 }
 
 __device__ float disney_pdf_trans(const BSDF& b, Vec3 lwi, Vec3 lwo) {
-    const float eta = lwo.z > 0 ? b.IOR : 1 / b.IOR;
+    const float eta = lwo.z > 0 ? b.dp->IOR : 1 / b.dp->IOR;
     Vec3 lwh = normalize(lwo + eta * lwi);
     if (lwh.z < 0) lwh = -lwh;
     if (((lwo.z > 0) != (dot(lwh, lwo) > 0)) || ((lwi.z > 0) != (dot(lwh, lwi) > 0))) return 0;
@@ -474,7 +471,7 @@ __device__ float disney_pdf_trans(const BSDF& b, Vec3 lwi, Vec3 lwo) {
     const float dwh_dwi = eta * eta * dot(lwi, lwh) / (sdem * sdem);
     float sph, cph;
     sincos_phi(lwh, &sph, &cph);
-    const float D = aniso_gtr2(sph, cph, cos_2_sin(lwh.z), lwh.z, b.trans_ax, b.trans_ay);
+    const float D = aniso_gtr2(sph, cph, cos_2_sin(lwh.z), lwh.z, b.dp->trans_ax, b.dp->trans_ay);
     return fabsf(lwh.z * D * dwh_dwi);
 }
 
@@ -532,22 +529,22 @@ __device__ __noinline__ BSDFValue bsdf_eval_pdf(const BSDF& b, Vec3 wi, Vec3 wo)
     // DisneyBSDF (disney.cpp:213-249, 328-401)
     if (fabsf(lwi.z) < b.eps || fabsf(lwo.z) < b.eps) return r;
     if (lwi.z < 0 || lwo.z < 0) {
-        if (b.transmission == 0.0f) return r;
+        if (b.dp->transmission == 0.0f) return r;
         const bool through = lwi.z * lwo.z < 0;
         r.f = (through ? disney_f_trans(b, lwi, lwo) : disney_f_inner(b, lwi, lwo)) * normal_corr(b, wi);
         if (lwo.z < 0) {
-            const float mF = clampf(dielectric_fresnel(b.IOR, 1, lwo.z), 0.1f, 0.9f);
+            const float mF = clampf(dielectric_fresnel(b.dp->IOR, 1, lwo.z), 0.1f, 0.9f);
             if (lwi.z > 0) {
                 r.pdf = (1 - mF) * disney_pdf_trans(b, lwi, lwo);
             } else {  // pdf_inner_refl (disney.cpp:386-401)
                 const Vec3 lwh = -normalize(lwi + lwo);
                 float sph, cph;
                 sincos_phi(lwh, &sph, &cph);
-                const float D = aniso_gtr2(sph, cph, cos_2_sin(lwh.z), lwh.z, b.trans_ax, b.trans_ay);
+                const float D = aniso_gtr2(sph, cph, cos_2_sin(lwh.z), lwh.z, b.dp->trans_ax, b.dp->trans_ay);
                 r.pdf = mF * fabsf(lwh.z * D / (4 * dot(lwi, lwh)));
             }
         } else {
-            r.pdf = b.w_transmission * disney_pdf_trans(b, lwi, lwo);
+            r.pdf = b.dp->w_transmission * disney_pdf_trans(b, lwi, lwo);
         }
         return r;
     }
@@ -555,43 +552,43 @@ __device__ __noinline__ BSDFValue bsdf_eval_pdf(const BSDF& b, Vec3 wi, Vec3 wo)
     const Vec3 lwh = normalize(lwi + lwo);
     const float cd = dot(lwi, lwh);
     Vec3 diffuse, sheen;
-    if (b.metallic < 1) {
+    if (b.dp->metallic < 1) {
         const float FL = one_minus_5(ci), FV = one_minus_5(co);
-        const float RR = 2 * b.roughness * cd * cd;
-        const Vec3 lam = b.C * kInvPi;
+        const float RR = 2 * b.dp->roughness * cd * cd;
+        const Vec3 lam = b.dp->C * kInvPi;
         diffuse = lam * (1 - 0.5f * FL) * (1 - 0.5f * FV) + lam * (RR * (FL + FV + FL * FV * (RR - 1)));
-        if (b.sheen > 0) sheen = 4 * b.sheen * mix(Vec3(1.0f), b.Ctint, b.sheen_tint) * one_minus_5(cd);
+        if (b.dp->sheen > 0) sheen = 4 * b.dp->sheen * mix(Vec3(1.0f), b.dp->Ctint, b.dp->sheen_tint) * one_minus_5(cd);
     }
     // f_specular (disney.cpp:213-249)
-    const Vec3 Cspec = mix(mix(Vec3(1.0f), b.Ctint, b.spec_tint), b.C, b.metallic);
+    const Vec3 Cspec = mix(mix(Vec3(1.0f), b.dp->Ctint, b.dp->spec_tint), b.dp->C, b.dp->metallic);
     const float fd = one_minus_5(cd);
-    const Vec3 diel = Cspec * dielectric_fresnel(b.IOR, 1, cd);
+    const Vec3 diel = Cspec * dielectric_fresnel(b.dp->IOR, 1, cd);
     const Vec3 cond = Cspec + (Vec3(1.0f) - Cspec) * fd;
-    const Vec3 F = mix(b.spec_scale * diel, cond, b.metallic);
+    const Vec3 F = mix(b.dp->spec_scale * diel, cond, b.dp->metallic);
     float sph, cph, spi, cpi, spo, cpo;
     sincos_phi(lwh, &sph, &cph);
     sincos_phi(lwi, &spi, &cpi);
     sincos_phi(lwo, &spo, &cpo);
     const float ch = lwh.z, sh = cos_2_sin(ch);
     const float ti = tan_theta(lwi), to = tan_theta(lwo);
-    const float D = aniso_gtr2(sph, cph, sh, ch, b.ax, b.ay);
-    const float G = smith_aniso_gtr2(cpi, spi, b.ax, b.ay, ti) * smith_aniso_gtr2(cpo, spo, b.ax, b.ay, to);
+    const float D = aniso_gtr2(sph, cph, sh, ch, b.dp->ax, b.dp->ay);
+    const float G = smith_aniso_gtr2(cpi, spi, b.dp->ax, b.dp->ay, ti) * smith_aniso_gtr2(cpo, spo, b.dp->ax, b.dp->ay, to);
     const Vec3 specular = F * (D * G / fabsf(4 * ci * co));
     // the clear coat's distribution serves its value and its density
-    const float Dc = gtr1(sh, ch, b.cc_rough);
+    const float Dc = gtr1(sh, ch, b.dp->cc_rough);
     Vec3 cc;
-    if (b.clearcoat > 0) {
+    if (b.dp->clearcoat > 0) {
         const float Fc = 0.04f + (1 - 0.04f) * fd;
         const float Gc = smith_gtr2(ti, 0.25f) * smith_gtr2(to, 0.25f);
-        cc = Vec3(b.clearcoat * Dc * Fc * Gc / fabsf(4 * ci * co));
+        cc = Vec3(b.dp->clearcoat * Dc * Fc * Gc / fabsf(4 * ci * co));
     }
-    const Vec3 value = (1 - b.metallic) * (1 - b.transmission) * (diffuse + sheen) + specular + cc;
+    const Vec3 value = (1 - b.dp->metallic) * (1 - b.dp->transmission) * (diffuse + sheen) + specular + cc;
     r.f = value * normal_corr(b, wi);
     // pdf_diffuse + pdf_specular_clearcoat (disney.cpp:328-356)
     spo = cos_2_sin(cpo);
-    const float ps = smith_aniso_gtr2(cpo, spo, b.ax, b.ay, to) * D / (4 * lwo.z);
+    const float ps = smith_aniso_gtr2(cpo, spo, b.dp->ax, b.dp->ay, to) * D / (4 * lwo.z);
     const float pc = ch * Dc / (4 * cd);
-    r.pdf = b.w_diffuse * zweighted_pdf(lwi.z) + b.w_specular * ps + b.w_clearcoat * pc;
+    r.pdf = b.dp->w_diffuse * zweighted_pdf(lwi.z) + b.dp->w_specular * ps + b.dp->w_clearcoat * pc;
     return r;
 }
 
@@ -751,12 +748,12 @@ __device__ BSDFSample bsdf_sample(const BSDF& b, Vec3 wo, float u0, float u1, fl
     Vec3 lwi;
     bool ok = false;
     if (lwo.z < 0) {
-        if (b.transmission == 0.0f) return r;
-        const float mF = clampf(dielectric_fresnel(b.IOR, 1, lwo.z), 0.1f, 0.9f);
+        if (b.dp->transmission == 0.0f) return r;
+        const float mF = clampf(dielectric_fresnel(b.dp->IOR, 1, lwo.z), 0.1f, 0.9f);
         if (u0 >= mF) {
             goto sample_trans;
         } else {
-            const Vec3 lwh = sample_aniso_gtr2(b.trans_ax, b.trans_ay, u1, u2);
+            const Vec3 lwh = sample_aniso_gtr2(b.dp->trans_ax, b.dp->trans_ay, u1, u2);
             if (lwh.z <= 0) return r;
             const Vec3 t = 2 * dot(lwo, lwh) * lwh - lwo;
             if (t.z > 0) return r;
@@ -768,24 +765,24 @@ __device__ BSDFSample bsdf_sample(const BSDF& b, Vec3 wo, float u0, float u1, fl
         // the diffuse choice is always overwritten (disney.cpp:578-589),
         // unless the fixed sampling mode is on
         float sel = u0;
-        if (b.disney_fixed && sel < b.w_diffuse) {
+        if (b.disney_fixed && sel < b.dp->w_diffuse) {
             float pdf;
             lwi = zweighted_on_hemisphere(u1, u2, &pdf);
             ok = lwi.z > 0;
             goto done;
         }
-        if (!(sel < b.w_diffuse)) sel -= b.w_diffuse;
-        if (sel < b.w_transmission) goto sample_trans;
-        sel -= b.w_transmission;
-        if (sel < b.w_specular) {
-            const Vec3 lwh = normalize(sample_gtr2_vnor(lwo, b.ax, b.ay, u1, u2, b.eps));
+        if (!(sel < b.dp->w_diffuse)) sel -= b.dp->w_diffuse;
+        if (sel < b.dp->w_transmission) goto sample_trans;
+        sel -= b.dp->w_transmission;
+        if (sel < b.dp->w_specular) {
+            const Vec3 lwh = normalize(sample_gtr2_vnor(lwo, b.dp->ax, b.dp->ay, u1, u2, b.eps));
             if (lwh.z <= 0) return r;
             const Vec3 t = normalize(2 * dot(lwo, lwh) * lwh - lwo);
             if (t.z <= 0) return r;
             lwi = t;
             ok = true;
         } else {
-            const Vec3 lwh = sample_gtr1(b.cc_rough, u1, u2);
+            const Vec3 lwh = sample_gtr1(b.dp->cc_rough, u1, u2);
             if (lwh.z <= 0) return r;
             const Vec3 t = normalize(2 * dot(lwo, lwh) * lwh - lwo);
             if (t.z <= 0) return r;
@@ -795,10 +792,10 @@ __device__ BSDFSample bsdf_sample(const BSDF& b, Vec3 wo, float u0, float u1, fl
         goto done;
     }
 sample_trans: {
-        const Vec3 lwh = sample_aniso_gtr2(b.trans_ax, b.trans_ay, u1, u2);
+        const Vec3 lwh = sample_aniso_gtr2(b.dp->trans_ax, b.dp->trans_ay, u1, u2);
         if (lwh.z <= 0) return r;
         if ((lwo.z > 0) != (dot(lwh, lwo) > 0)) return r;
-        const float eta = lwo.z > 0 ? 1 / b.IOR : b.IOR;
+        const float eta = lwo.z > 0 ? 1 / b.dp->IOR : b.dp->IOR;
         const Vec3 owh = dot(lwh, lwo) > 0 ? lwh : -lwh;
         const float ci = dot(lwo, owh);
         const float s2t = sqrf(eta) * (1 - sqrf(ci));
@@ -879,7 +876,10 @@ __device__ __forceinline__ float nd_scale(float a) {
 }
 
 // Material::shade
-__device__ BSDF shade(const Scene& S, const Surface& s, Vec3* shading_normal) {
+// `own` holds the Disney parameters of a vertex whose material has textures;
+// a constant material's were computed with the scene (k_disney_params), and
+// every vertex on it reads that one copy.
+__device__ BSDF shade(const Scene& S, const Surface& s, Vec3* shading_normal, DisneyParams* own) {
     const Entity& e = S.entities[s.entity];
     const Material& m = S.materials[e.material];
     BSDF b;
@@ -917,15 +917,17 @@ __device__ BSDF shade(const Scene& S, const Surface& s, Vec3* shading_normal) {
         b.albedo = m.all_constant ? Vec3(m.c[0], m.c[1], m.c[2]) : tv[0];
     } else if (m.type == ATRC_MAT_DISNEY) {
         if (m.all_constant) {
-            disney_init(b, Vec3(m.c[0], m.c[1], m.c[2]), m.c[3], m.c[4], m.c[5], m.c[6], m.c[7],
-                        Vec3(m.c[8], m.c[9], m.c[10]), m.c[11], m.c[12], m.c[13], m.c[14], m.c[15], m.cc_gloss);
+            b.dp = S.disney + e.material;
+            b.albedo = Vec3(m.c[0], m.c[1], m.c[2]);
         } else {
             auto T = [&](int slot) { return tv[slot]; };
-            disney_init(b, T(ATRC_DISNEY_BASE_COLOR), T(ATRC_DISNEY_METALLIC).x, T(ATRC_DISNEY_ROUGHNESS).x,
+            disney_init(*own, T(ATRC_DISNEY_BASE_COLOR), T(ATRC_DISNEY_METALLIC).x, T(ATRC_DISNEY_ROUGHNESS).x,
                         T(ATRC_DISNEY_TRANSMISSION).x, T(ATRC_DISNEY_TRANSMISSION_ROUGHNESS).x, T(ATRC_DISNEY_IOR).x,
                         T(ATRC_DISNEY_SPECULAR_SCALE), T(ATRC_DISNEY_SPECULAR_TINT).x, T(ATRC_DISNEY_ANISOTROPIC).x,
                         T(ATRC_DISNEY_SHEEN).x, T(ATRC_DISNEY_SHEEN_TINT).x, T(ATRC_DISNEY_CLEARCOAT).x,
                         T(ATRC_DISNEY_CLEARCOAT_GLOSS).x);
+            b.dp = own;
+            b.albedo = T(ATRC_DISNEY_BASE_COLOR);
         }
     } else if (m.type == ATRC_MAT_MIRROR || m.type == ATRC_MAT_GLASS || m.type == ATRC_MAT_METAL ||
                m.type == ATRC_MAT_PHONG) {

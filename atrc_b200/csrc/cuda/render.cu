@@ -333,6 +333,18 @@ struct Pool {
 };
 constexpr int kShadowKeys = 4096;  // 16 x 16 x 16 origin cells
 
+// Disney parameters of the constant Disney materials, once per scene.
+__global__ void k_disney_params(const Material* materials, int n, DisneyParams* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const Material& m = materials[i];
+    if (m.type != ATRC_MAT_DISNEY || !m.all_constant) return;
+    DisneyParams p;
+    disney_init(p, Vec3(m.c[0], m.c[1], m.c[2]), m.c[3], m.c[4], m.c[5], m.c[6], m.c[7], Vec3(m.c[8], m.c[9], m.c[10]),
+                m.c[11], m.c[12], m.c[13], m.c[14], m.c[15], m.cc_gloss);
+    out[i] = p;
+}
+
 // End of one window of the device-side bounce loop: run another window
 // unless the work is done or a watchdog fired; after max_windows the loop
 // stops with kWatchdogLoop instead of running on (no path lives that long).
@@ -1205,7 +1217,7 @@ __device__ __forceinline__ bool subsurface_sample(const Scene& S, const Material
     b.type = kMatSeparable;
     b.geo = x->geo;
     b.shd = x->geo;
-    b.IOR = eta;
+    b.glass_ior = eta;
     b.sep_ci = 1.0f - 2.0f * fresnel_moment1(1.0f / eta);
     b.eps = eps;
     *bx = b;
@@ -1232,12 +1244,13 @@ __global__ void k_guide_features(Scene S, Params p, Pool P, Counters* c) {
         if (ent >= 0 && !(flags & PF_TERMINATE) && (p.gf.max_depth <= 0 || depth <= p.gf.max_depth)) {
             const Surface s = make_surface(S, h, xyz(ray), xyz2(ray));
             Vec3 sn;
-            const BSDF b = shade(S, s, &sn);
+            DisneyParams own;
+            const BSDF b = shade(S, s, &sn, &own);
             if (guidable(S.materials[S.entities[ent].material]) && !fringes(b, s.wr)) {
                 q.pos[0] = s.pos.x; q.pos[1] = s.pos.y; q.pos[2] = s.pos.z;
                 q.nrm[0] = sn.x; q.nrm[1] = sn.y; q.nrm[2] = sn.z;
                 q.wo[0] = s.wr.x; q.wo[1] = s.wr.y; q.wo[2] = s.wr.z;
-                q.rough = b.type == ATRC_MAT_DISNEY || b.type == ATRC_MAT_METAL ? b.roughness : 1.0f;
+                q.rough = b.type == ATRC_MAT_DISNEY ? b.dp->roughness : b.type == ATRC_MAT_METAL ? b.roughness : 1.0f;
                 q.slot = slot;
             }
         }
@@ -1354,7 +1367,8 @@ __global__ void __launch_bounds__(128, ATRC_SHADE_MIN_BLOCKS) k_shade(Scene S, P
         if (!finish) {
             const Entity& e = S.entities[ent];
             Vec3 sn;
-            const BSDF b = shade(S, s, &sn);
+            DisneyParams own;
+            const BSDF b = shade(S, s, &sn, &own);
             if (depth == 1 && p.gbuffer) {
                 const Vec3 alb = bsdf_albedo(b);
                 P.gb_albedo[slot] = make_float4(alb.x, alb.y, alb.z, (e.flags & ENT_NO_DENOISE) ? 0.0f : 1.0f);
@@ -1789,7 +1803,7 @@ struct DeviceSceneImpl {
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     Scene scene{};
-    DevBuf nodes, tris, tri_bc, tri_shade, tri_orig, entities, tlas_order, materials, tex2d, tex3d, texels, media, alias_prob,
+    DevBuf nodes, tris, tri_bc, tri_shade, tri_orig, entities, tlas_order, materials, disney, tex2d, tex3d, texels, media, alias_prob,
         alias_idx, env_probs, env_alias_prob, env_alias_idx;
     DevBuf watchdog;
     DevBuf tiles;  // tile tables of the film's sample grid
@@ -2181,6 +2195,13 @@ int atrc_cuda_scene_create(const AtrcSceneDesc* desc, AtrcScene** out) {
         S.tlas_order = upload(d.tlas_order, hs->tlas_order, s);
         S.materials = upload(d.materials, hs->materials, s);
         S.material_count = int32_t(hs->materials.size());
+        if (S.material_count > 0) {
+            d.disney.alloc(hs->materials.size() * sizeof(DisneyParams));
+            k_disney_params<<<(S.material_count + 127) / 128, 128, 0, s>>>(S.materials, S.material_count,
+                                                                         d.disney.as<DisneyParams>());
+            CK(cudaGetLastError());
+            S.disney = d.disney.as<DisneyParams>();
+        }
         S.tex2d = upload(d.tex2d, hs->tex2d, s);
         S.tex3d = upload(d.tex3d, hs->tex3d, s);
         S.texels = upload(d.texels, hs->texels, s);
