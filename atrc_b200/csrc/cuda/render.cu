@@ -333,6 +333,115 @@ struct Pool {
 };
 constexpr int kShadowKeys = 4096;  // 16 x 16 x 16 origin cells
 
+// ------------------------------------------------------ top-level bounds
+// An instance's bound in the top-level tree comes from the eight transformed
+// corners of its mesh's box (transform_wrapper.cpp:13-27): a rotated sphere's
+// is up to 1.7 times as wide as the sphere, and rays that only cross the
+// corners enter its tree for nothing.  With the scene, k_instance_bounds takes
+// the transformed vertices instead, and k_refit_tlas shrinks the top-level
+// boxes to them; the bounds are widened by far more than the transforms round,
+// so hits do not change (scene bound and environment keep the corner boxes).
+// 64 instances: 4M incoherent queries 1.76 -> 1.58 ms, the instanced frame
+// 30.6 -> 29.0, ao 3.50 -> 3.36.
+__device__ __forceinline__ uint32_t order_bits(float x) {  // unsigned order = float order
+    const uint32_t b = __float_as_uint(x);
+    return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float from_order_bits(uint32_t b) {
+    return __uint_as_float(b & 0x80000000u ? b & 0x7fffffffu : ~b);
+}
+
+// Triangles whose vertices say where the instance is (baked into mesh space).
+__device__ __forceinline__ bool tight_bound(const Entity& e) {
+    return e.kind == LEAF_TRIANGLES && (e.flags & ENT_WRAP) && !(e.flags & ENT_LOCAL);
+}
+
+// grid (blocks per entity, entities); bounds: per entity lo xyz (start at
+// ~0), hi xyz (start at 0) as order_bits.
+__global__ void __launch_bounds__(256) k_instance_bounds(Scene S, uint32_t* bounds) {
+    for (int ei = blockIdx.y; ei < S.entity_count; ei += gridDim.y) {
+        const Entity& e = S.entities[ei];
+        if (!tight_bound(e)) continue;
+        Vec3 lo(INFINITY), hi(-INFINITY);
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < e.tri_count; t += gridDim.x * blockDim.x) {
+            const float4* tp = reinterpret_cast<const float4*>(S.tris) + size_t(e.tri_first + t) * 3;
+            const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+            const Vec3 A(a.x, a.y, a.z);
+            const Vec3 v[3] = {A, A + Vec3(b.x, b.y, b.z), A + Vec3(c.x, c.y, c.z)};
+            for (int k = 0; k < 3; ++k) {
+                const Vec3 w = apply_point_rn(e.wrap_m, v[k]);
+                lo = Vec3(fminf(lo.x, w.x), fminf(lo.y, w.y), fminf(lo.z, w.z));
+                hi = Vec3(fmaxf(hi.x, w.x), fmaxf(hi.y, w.y), fmaxf(hi.z, w.z));
+            }
+        }
+        const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+        for (int a = 0; a < 3; ++a) {
+            const uint32_t ml = __reduce_min_sync(0xffffffffu, order_bits(l[a]));
+            const uint32_t mh = __reduce_max_sync(0xffffffffu, order_bits(h[a]));
+            if ((threadIdx.x & 31) == 0) {
+                atomicMin(bounds + 6 * ei + a, ml);
+                atomicMax(bounds + 6 * ei + 3 + a, mh);
+            }
+        }
+    }
+}
+
+// Child k's box of a wide node, as three pairs of floats.
+__device__ __forceinline__ float* box_lo(Bvh4Node* n, int axis) { return reinterpret_cast<float*>(n) + 8 * axis; }
+__device__ __forceinline__ float* box_hi(Bvh4Node* n, int axis) { return reinterpret_cast<float*>(n) + 8 * axis + 4; }
+
+// One block: the leaves' boxes, then `depth` rounds in which every node takes
+// its interior children's boxes from their nodes (boxes only shrink, and after
+// as many rounds as the tree has levels none changes).
+__global__ void __launch_bounds__(256) k_refit_tlas(Scene S, Bvh4Node* nodes, int first, int count, int depth,
+                                                   const uint32_t* bounds) {
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        Bvh4Node* n = nodes + first + i;
+        for (int k = 0; k < 4; ++k) {
+            const int32_t link = n->link[k];
+            if (link >= 0 || link == kEmptyLink) continue;
+            const uint32_t enc = uint32_t(~link);
+            if ((enc & 15) != 0) continue;  // one entity per leaf
+            const int ei = int(S.tlas_order[enc >> 4]);
+            if (!tight_bound(S.entities[ei])) continue;
+            for (int a = 0; a < 3; ++a) {
+                const float lo = from_order_bits(bounds[6 * ei + a]), hi = from_order_bits(bounds[6 * ei + 3 + a]);
+                if (!(lo <= hi)) continue;  // no finite vertex
+                const float pad = 1e-5f * fmaxf(fabsf(lo), fabsf(hi)) + 1e-4f * (hi - lo);
+                float *bl = box_lo(n, a) + k, *bh = box_hi(n, a) + k;
+                *bl = fmaxf(*bl, lo - pad);
+                *bh = fminf(*bh, hi + pad);
+            }
+        }
+    }
+    for (int round = 0; round < depth; ++round) {
+        __threadfence_block();
+        __syncthreads();
+        for (int i = threadIdx.x; i < count; i += blockDim.x) {
+            Bvh4Node* n = nodes + first + i;
+            for (int k = 0; k < 4; ++k) {
+                const int32_t link = n->link[k];
+                if (link < 0) continue;
+                Bvh4Node* m = nodes + link;
+                for (int a = 0; a < 3; ++a) {
+                    float lo = INFINITY, hi = -INFINITY;
+                    for (int j = 0; j < 4; ++j) {
+                        if (m->link[j] == kEmptyLink) continue;
+                        lo = fminf(lo, reinterpret_cast<volatile float*>(box_lo(m, a))[j]);
+                        hi = fmaxf(hi, reinterpret_cast<volatile float*>(box_hi(m, a))[j]);
+                    }
+                    box_lo(n, a)[k] = lo;
+                    box_hi(n, a)[k] = hi;
+                }
+            }
+        }
+    }
+}
+
+// Triangles over all instances up to which their bounds are taken (48 bytes
+// each, once per scene: 2^28 are about 3 ms).
+constexpr size_t kTightTriangles = size_t(1) << 28;
+
 // Disney parameters of the constant Disney materials, once per scene.
 __global__ void k_disney_params(const Material* materials, int n, DisneyParams* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2254,6 +2363,22 @@ int atrc_cuda_scene_create(const AtrcSceneDesc* desc, AtrcScene** out) {
         S.env.alias_prob = upload(d.env_alias_prob, hs->env_alias_prob, s);
         S.env.alias_idx = upload(d.env_alias_idx, hs->env_alias_idx, s);
         S.eps = 3e-4f;
+        size_t instanced = 0;
+        for (const Entity& e : hs->entities) instanced += e.flags & ENT_WRAP ? size_t(e.tri_count) : 0;
+        DevBuf bounds;
+        if (instanced > 0 && instanced <= kTightTriangles && S.tlas_root >= 0) {
+            const size_t ne = hs->entities.size();
+            std::vector<uint32_t> start(6 * ne, 0u);
+            for (size_t k = 0; k < ne; ++k)
+                for (int a = 0; a < 3; ++a) start[6 * k + a] = ~0u;
+            uint32_t* db = const_cast<uint32_t*>(upload(bounds, start, s));
+            const int blocks = std::max(1, int(d.sm_count * 8 / std::min<size_t>(ne, 1024)));
+            k_instance_bounds<<<dim3(blocks, unsigned(std::min<size_t>(ne, 65535))), 256, 0, s>>>(S, db);
+            k_refit_tlas<<<1, 256, 0, s>>>(S, d.nodes.as<Bvh4Node>(), int(hs->tlas_first),
+                                           int(hs->nodes.size() - hs->tlas_first), hs->tlas_depth + 1, db);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(s));  // `start` and `bounds` end with this scope
+        }
         d.scene = S;
         d.choose_default_sort(hs->entities, hs->materials);
         d.shadow_warps = hs->tri_orig.size() >= kShadowWarps;

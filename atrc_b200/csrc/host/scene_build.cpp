@@ -412,6 +412,7 @@ void build_host_scene(const AtrcSceneDesc& d, HostScene* hs, int device) {
         }
         BvhResult tl = build_bvh(eprims, 1);  // one entity per top-level leaf
         hs->tlas_depth = tl.max_depth;
+        hs->tlas_first = hs->nodes.size();
         hs->scene.tlas_root = collapse_bvh4(tl, &hs->nodes);
         validate_bvh4(hs->nodes, hs->scene.tlas_root, 0, uint32_t(d.entity_count));
         hs->tlas_order = tl.order;

@@ -31,6 +31,7 @@ struct HostScene {
     std::vector<int32_t> env_alias_idx;
     dev::Scene scene{};               // pointers left null; filled on upload
     int max_blas_depth = 0, tlas_depth = 0;
+    size_t tlas_first = 0;  // the top-level tree's nodes are nodes[tlas_first ...]
 };
 
 // Throws std::runtime_error with a message on unsupported or invalid input.
