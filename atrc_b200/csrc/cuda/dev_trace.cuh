@@ -9,7 +9,11 @@
 // Moller-Trumbore test (src/tracer/include/agz/tracer/utility/
 // triangle_aux.h:9-69).  The intersection mode (IsectMode) is a template
 // parameter of the traversal:
-//   ISECT_FAST       Moller-Trumbore as the compiler schedules it (FMAs);
+//   ISECT_FAST       Moller-Trumbore with fused multiply-adds, written out so
+//                    that every kernel and register budget decides an edge
+//                    alike (left to the compiler, alpha + beta was fused in
+//                    some kernels and not in others, and one ray in about ten
+//                    million met an edge in one and missed it in the other);
 //   ISECT_EXACT      every float operation of the ray transform and of
 //                    Moller-Trumbore in the reference's order without fused
 //                    multiply-adds, so hit distances are bit-identical;
@@ -72,6 +76,15 @@ __device__ __forceinline__ Vec3 safe_inv(Vec3 d) { return Vec3(safe_rcp(d.x), sa
 
 enum IsectMode : int { ISECT_FAST = 0, ISECT_EXACT = 1, ISECT_WATERTIGHT = 2 };
 
+// Cross and dot product with their fused multiply-adds written out.
+__device__ __forceinline__ Vec3 cross_fma(Vec3 a, Vec3 b) {
+    return Vec3(__fmaf_rn(a.y, b.z, -__fmul_rn(a.z, b.y)), __fmaf_rn(a.z, b.x, -__fmul_rn(a.x, b.z)),
+                __fmaf_rn(a.x, b.y, -__fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ float dot_fma(Vec3 a, Vec3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+
 // Moller-Trumbore.  ANY selects has_intersection_with_triangle (alpha <= 1
 // also checked), otherwise closest_intersection_with_triangle.
 template <bool EXACT, bool ANY>
@@ -96,17 +109,17 @@ __device__ __forceinline__ bool mt_test(const RayState& r, const float4& p0, con
         *v_out = beta;
         return true;
     } else {
-        const Vec3 s1 = cross(r.d, C_A);
-        const float div = dot(s1, B_A);
+        const Vec3 s1 = cross_fma(r.d, C_A);
+        const float div = dot_fma(s1, B_A);
         if (div == 0.0f) return false;
-        const float inv_div = 1.0f / div;
-        const Vec3 o_A = r.o - A;
-        const float alpha = dot(o_A, s1) * inv_div;
+        const float inv_div = __fdiv_rn(1.0f, div);
+        const Vec3 o_A = sub_rn(r.o, A);
+        const float alpha = __fmul_rn(dot_fma(o_A, s1), inv_div);
         if (alpha < 0 || (ANY && alpha > 1)) return false;
-        const Vec3 s2 = cross(o_A, B_A);
-        const float beta = dot(r.d, s2) * inv_div;
-        if (beta < 0 || alpha + beta > 1) return false;
-        const float t = dot(C_A, s2) * inv_div;
+        const Vec3 s2 = cross_fma(o_A, B_A);
+        const float db = dot_fma(r.d, s2), beta = __fmul_rn(db, inv_div);
+        if (beta < 0 || (ANY ? __fmaf_rn(db, inv_div, alpha) : __fadd_rn(alpha, beta)) > 1) return false;
+        const float t = __fmul_rn(dot_fma(C_A, s2), inv_div);
         if (!(r.tmin <= t && t <= tmax)) return false;
         *t_out = t;
         *u_out = alpha;

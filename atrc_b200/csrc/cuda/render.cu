@@ -53,7 +53,7 @@
 #define ATRC_TRACE_MIN_BLOCKS 8  // the same for the traversal kernels
 #endif
 #ifndef ATRC_SHADOW_MIN_BLOCKS
-#define ATRC_SHADOW_MIN_BLOCKS 10  // k_shadow: 48 registers (8 blocks, 64 registers, measured 2-6 % slower)
+#define ATRC_SHADOW_MIN_BLOCKS 9  // k_shadow: 56 registers (10 blocks, 48 registers: room 9.65 against 8.16 ms; 8 blocks the same)
 #endif
 
 namespace atrc {
@@ -1746,9 +1746,10 @@ __device__ __forceinline__ void shadow_ray(const Scene& S, Pool& P, Counters* c,
 // their first by their place in the grid and the next from a cursor, so that no
 // block waits for its slowest warp; else one ray per thread of a grid that
 // covers the queue.  In large scenes, whose rays differ most in length, the
-// warps win (occlusion rays of the room 10.1 -> 9.7 ms, of ao on the instanced
-// scene 2.15 -> 2.02, of the guided room 3.08 -> 2.91), in small ones the
-// blocks (Cornell 1.68 against 1.78, media 0.76 against 1.02): kShadowWarps.
+// warps win (with 48 registers, occlusion rays of the room 10.1 -> 9.7 ms, of
+// ao on the instanced scene 2.15 -> 2.02, of the guided room 3.08 -> 2.91), in
+// small ones the blocks (Cornell 1.68 against 1.78, media 0.76 against 1.02):
+// kShadowWarps.
 template <int ISECT, bool COUNT, bool WARPS>
 __global__ void __launch_bounds__(kTraceBlock, ATRC_SHADOW_MIN_BLOCKS) k_shadow(Scene S, Pool P, Counters* c) {
     if (!P.shadow_sort) mark_stage(c, 2);
@@ -2094,7 +2095,7 @@ struct PoolLayout {
 // k_shadow's grid.  The queue's length is known only on the device, so the
 // grid is fixed when the window is captured; k_shadow strides over the queue
 // and a thread traces one ray as long as the queue holds at most
-// kShadowGridWaves resident waves (148 SMs x 10 blocks x 128 threads each).
+// kShadowGridWaves resident waves (148 SMs x 9 blocks x 128 threads each).
 // A grid covering the whole capacity (the pool times the rays one path can
 // emit) would launch tens of thousands of blocks that find no ray: an
 // iteration of the instanced workload queues about 260,000 occlusion rays
