@@ -280,7 +280,7 @@ constexpr uint32_t kTrTmemCols = 512;
 struct TrainArgs {
     const GuideRecord* rec;
     int n;                     // records in this batch
-    const float* weight_sum;   // sum of the batch's targets (device)
+    const double* weight_sum;  // sum of the batch's targets (device)
     float* grad_w;             // FP32 gradients of the packed weights
     float* grad_table;         // FP32 gradients of the table
     float* loss;               // sum of the batch's loss terms
@@ -378,10 +378,11 @@ __global__ void __launch_bounds__(kTile, 1) k_guide_train(NetView net, TrainArgs
     tc::fence_after_sync();
     const uint32_t tm = *tslot;
     auto S = [&](int off) { return tc::smem_addr(smem + off); };
-    const float inv_wsum = *a.weight_sum > 0 ? 1.0f / *a.weight_sum : 0.0f;
+    const float wsum = float(*a.weight_sum);
+    const float inv_wsum = wsum > 0 ? 1.0f / wsum : 0.0f;
     // a few records of a batch can carry most of its weight (a path that found
     // the light): capping the targets keeps one step from following them alone
-    const float tcap = a.target_clamp > 0.0f ? a.target_clamp * *a.weight_sum / float(max(a.n, 1)) : INFINITY;
+    const float tcap = a.target_clamp > 0.0f ? a.target_clamp * wsum / float(max(a.n, 1)) : INFINITY;
     uint32_t phase = 0;
     const int t = threadIdx.x;
     bool first = true, ok = true;
@@ -525,8 +526,12 @@ __global__ void k_mix_pdf(const float* __restrict__ mixes, const float* __restri
     }
 }
 
-__global__ void k_target_sum(const GuideRecord* rec, int n, float* sum) {
-    float s = 0;
+// In 64 bits: the order in which the warps add no longer shows in the sum's
+// last bits, and with them in every weight of the batch and in the BF16
+// rounding of its gradients (gradients of the same batch differed by up to 2e-4
+// from run to run).
+__global__ void k_target_sum(const GuideRecord* rec, int n, double* sum) {
+    double s = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += rec[i].target;
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(sum, s);
@@ -934,13 +939,15 @@ int atrc_guide_pdf(AtrcGuide* g, const float* queries, const float* dirs, size_t
 // One Adam step on `n` records at `records` (device) -- internal helper.
 static void train_step(GuideImpl& G, const GuideRecord* rec, int n, float* loss_out) {
     cudaStream_t s = G.stream;
-    float* sc = G.scratch.as<float>();  // [0] target sum, [1] loss
-    CK(cudaMemsetAsync(sc, 0, 2 * sizeof(float), s));
-    k_target_sum<<<G.sm_count * 2, 256, 0, s>>>(rec, n, sc);
+    float* sc = G.scratch.as<float>();  // [1] loss, [4] live records, [8, 9] target sum in 64 bits
+    double* wsum = reinterpret_cast<double*>(sc + 8);
+    CK(cudaMemsetAsync(sc + 1, 0, sizeof(float), s));
+    CK(cudaMemsetAsync(wsum, 0, sizeof(double), s));
+    k_target_sum<<<G.sm_count * 2, 256, 0, s>>>(rec, n, wsum);
     TrainArgs a;
     a.rec = rec;
     a.n = n;
-    a.weight_sum = sc;
+    a.weight_sum = wsum;
     a.grad_w = G.w_g.as<float>();
     a.grad_table = G.t_g.as<float>();
     a.loss = sc + 1;
@@ -1042,15 +1049,17 @@ int atrc_guide_gradients(AtrcGuide* g, const float* records, size_t n, float* gr
         cudaStream_t s = G.stream;
         CK(cudaMemcpyAsync(G.records.p, records, n * sizeof(GuideRecord), cudaMemcpyHostToDevice, s));
         float* sc = G.scratch.as<float>();
-        CK(cudaMemsetAsync(sc, 0, 2 * sizeof(float), s));
+        double* wsum = reinterpret_cast<double*>(sc + 8);
+        CK(cudaMemsetAsync(sc + 1, 0, sizeof(float), s));
+        CK(cudaMemsetAsync(wsum, 0, sizeof(double), s));
         CK(cudaMemsetAsync(G.w_g.p, 0, kWeights * sizeof(float), s));
         CK(cudaMemsetAsync(G.t_g.p, 0, G.table_n * sizeof(float), s));
         const GuideRecord* rec = G.records.as<GuideRecord>();
-        k_target_sum<<<G.sm_count * 2, 256, 0, s>>>(rec, int(n), sc);
+        k_target_sum<<<G.sm_count * 2, 256, 0, s>>>(rec, int(n), wsum);
         TrainArgs a;
         a.rec = rec;
         a.n = int(n);
-        a.weight_sum = sc;
+        a.weight_sum = wsum;
         a.grad_w = G.w_g.as<float>();
         a.grad_table = G.t_g.as<float>();
         a.loss = sc + 1;
