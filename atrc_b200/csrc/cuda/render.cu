@@ -1021,7 +1021,7 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend(S
     bool cont = CONT && n_cont > 0;
     int a0 = 0, a1 = 0, b0 = 0, b1 = 0;  // reserved entries of the free-slot list
     for (;;) {
-        const bool old = CONT && cont;  // this round's rays are continuations (warp-uniform)
+        const bool old = CONT && cont;  // the 32 rays to trace next are continuations (warp-uniform)
         int i, slot = 0;
         bool active;
         CameraSample cs;
@@ -1055,7 +1055,7 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend(S
                     break;
                 }
             }
-            // every claimed sample is traced in this round: none is lost when
+            // every claimed sample is traced at once: none is lost when
             // the slots run out
             const int m = min(32, have);
             int base = 0;

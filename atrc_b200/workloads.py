@@ -24,6 +24,10 @@ from __future__ import annotations
 import argparse
 
 
+def _seen(percent: float) -> None:
+    pass
+
+
 def instanced(spp: int, warmup: int, steps: int) -> None:
     import torch
 
@@ -38,7 +42,7 @@ def instanced(spp: int, warmup: int, steps: int) -> None:
         desc.first_spp = k * spp
         if k >= warmup:
             torch.cuda.nvtx.range_push("step")
-        stats = scene.render(desc, film)
+        stats = scene.render(desc, film, progress=_seen)
         if k >= warmup:
             torch.cuda.synchronize()
             torch.cuda.nvtx.range_pop()
@@ -56,7 +60,7 @@ def subsurface(spp: int, warmup: int, steps: int) -> None:
     desc.spp_count = spp
     for k in range(warmup + steps):
         desc.first_spp = k * spp
-        stats = scene.render(desc, film)
+        stats = scene.render(desc, film, progress=_seen)
         torch.cuda.synchronize()
         if k >= warmup:
             print(f"step {k - warmup}: closest rays {stats['rays_closest']}, shadow rays {stats['rays_shadow']}")
@@ -74,7 +78,7 @@ def ploc() -> None:
     desc, _ = cfg.rendering(0)
     scene = DeviceScene(cfg)
     desc.spp_count = 1
-    stats = scene.render(desc, Film(desc.width, desc.height, device=True))
+    stats = scene.render(desc, Film(desc.width, desc.height, device=True), progress=_seen)
     print(f"closest rays {stats['rays_closest']}")
 
 

@@ -201,8 +201,9 @@ def reference_arm(args, rank: int, world: int) -> None:
 # DRAM bytes per closest ray of k_extend on the instanced workload, from one
 # ncu capture of every k_extend launch of an NVTX-marked 2-spp step
 # (dram__bytes_read.sum + dram__bytes_write.sum summed over the launches,
-# divided by the step's closest rays: 1,247.9 MB / 5,306,689 rays).
-K_EXTEND_DRAM_BYTES_PER_RAY = 235.2
+# divided by the step's closest rays: 1,571.9 MB / 5,305,924 rays; the kernel
+# makes the camera rays, writes new paths and splats the misses, too).
+K_EXTEND_DRAM_BYTES_PER_RAY = 296.2
 
 
 def stream_read_peaks(device: int) -> dict:
@@ -447,7 +448,7 @@ def batch_comparison(args) -> dict:
                "batched": {"seconds": t_batch, "Msamples_per_s": samples / t_batch / 1e6, "completion": q(secs),
                            "loop": "one graph launch: device-side WHILE node, per-view device timestamps"},
                "one_by_one": {"seconds": t_one, "Msamples_per_s": samples / t_one / 1e6, "completion": q(one_secs),
-                              "loop": "atrc_cuda_render_guided per view (windowed graph, host polls)"},
+                              "loop": "atrc_cuda_render_guided per view"},
                "speedup": t_one / t_batch}
         if device_loop_one_by_one:
             # the same views one by one through the device-side loop: what

@@ -352,9 +352,11 @@ typedef struct AtrcRenderStats {
     uint64_t iterations;       /* wavefront iterations                       */
     uint64_t kernel_launches;  /* kernels launched by this call              */
     uint64_t watchdog_flags;   /* device loops that hit their caps           */
-    double   extend_seconds;   /* device time inside closest-hit kernels     */
-    double   shadow_seconds;   /* device time inside any-hit kernels         */
-    double   shade_seconds;    /* device time inside shading kernels         */
+    /* device time of the stages, from the start of a stage's first kernel to
+     * the start of the next stage's (%globaltimer) */
+    double   extend_seconds;   /* camera rays and closest hits, material sort */
+    double   shadow_seconds;   /* any-hit kernels                            */
+    double   shade_seconds;    /* shading, guide and subsurface kernels      */
     uint64_t h2d_bytes, d2h_bytes;
     uint64_t extend_launches;  /* closest-hit kernel launches               */
     uint64_t shadow_launches;  /* any-hit kernel launches                   */
@@ -497,8 +499,8 @@ int atrc_cuda_render(AtrcScene* scene, const AtrcRenderDesc* desc,
 typedef struct AtrcTuning {
     int32_t path_pool;          /* paths in flight (queue capacity)              */
     int32_t sort_mode;          /* AtrcSortMode, never ATRC_SORT_AUTO            */
-    int32_t gen_blocks_per_sm;  /* grid of the generate / finish kernels per SM  */
-    int32_t gen_threads;        /* block size of the camera-ray generator        */
+    int32_t gen_blocks_per_sm;  /* grid of the slot-scan / finish kernels per SM */
+    int32_t gen_threads;        /* block size of the slot scan                   */
     int32_t finish_threads;     /* block size of the film splat                  */
     int32_t trials;             /* trial renders measured by the last autotune   */
     double  ms_per_msample;     /* device ms per million samples, chosen config  */
@@ -725,7 +727,7 @@ int  atrc_guide_gradients(AtrcGuide* guide, const float* records, size_t n,
  * must hold device pointers.  `guide` may be NULL (plain) or a trained guide
  * (sampling only).  view_seconds (may be NULL) receives per view the time,
  * on the device's global timer, from the start of the render to the splat of
- * the view's last sample.  `stats` has counts but no per-kernel timings.
+ * the view's last sample.
  * At most 1024 views. */
 int  atrc_cuda_render_batch(AtrcScene* scene, AtrcGuide* guide,
                             const AtrcRenderDesc* views, int32_t n,
