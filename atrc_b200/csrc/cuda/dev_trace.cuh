@@ -10,10 +10,12 @@
 // triangle_aux.h:9-69).  The intersection mode (IsectMode) is a template
 // parameter of the traversal:
 //   ISECT_FAST       Moller-Trumbore with fused multiply-adds, written out so
-//                    that every kernel and register budget decides an edge
-//                    alike (left to the compiler, alpha + beta was fused in
-//                    some kernels and not in others, and one ray in about ten
-//                    million met an edge in one and missed it in the other);
+//                    that a change of registers or of the code around it does
+//                    not move an edge.  The edge alpha + beta <= 1 has two
+//                    forms (FUSED_EDGE): occlusion rays of renders fuse one
+//                    product into the sum, all other rays round both terms
+//                    first, so of some hundred million random rays one meets
+//                    an edge as one kind and misses it as the other;
 //   ISECT_EXACT      every float operation of the ray transform and of
 //                    Moller-Trumbore in the reference's order without fused
 //                    multiply-adds, so hit distances are bit-identical;
@@ -86,8 +88,12 @@ __device__ __forceinline__ float dot_fma(Vec3 a, Vec3 b) {
 }
 
 // Moller-Trumbore.  ANY selects has_intersection_with_triangle (alpha <= 1
-// also checked), otherwise closest_intersection_with_triangle.
-template <bool EXACT, bool ANY>
+// also checked), otherwise closest_intersection_with_triangle.  FUSED_EDGE:
+// alpha + beta as fma(alpha's dividend, 1 / div, beta).  Which form a kernel
+// takes is part of its results: either is as good, but with the other one a
+// path whose occlusion ray grazes an edge takes another value (the indoor room
+// at 1280x720, 4 spp: a pixel in one image of five).
+template <bool EXACT, bool ANY, bool FUSED_EDGE>
 __device__ __forceinline__ bool mt_test(const RayState& r, const float4& p0, const float4& p1, const float4& p2,
                                         float tmax, float* t_out, float* u_out, float* v_out) {
     const Vec3 A(p0.x, p0.y, p0.z), B_A(p1.x, p1.y, p1.z), C_A(p2.x, p2.y, p2.z);
@@ -114,11 +120,11 @@ __device__ __forceinline__ bool mt_test(const RayState& r, const float4& p0, con
         if (div == 0.0f) return false;
         const float inv_div = __fdiv_rn(1.0f, div);
         const Vec3 o_A = sub_rn(r.o, A);
-        const float alpha = __fmul_rn(dot_fma(o_A, s1), inv_div);
+        const float da = dot_fma(o_A, s1), alpha = __fmul_rn(da, inv_div);
         if (alpha < 0 || (ANY && alpha > 1)) return false;
         const Vec3 s2 = cross_fma(o_A, B_A);
-        const float db = dot_fma(r.d, s2), beta = __fmul_rn(db, inv_div);
-        if (beta < 0 || (ANY ? __fmaf_rn(db, inv_div, alpha) : __fadd_rn(alpha, beta)) > 1) return false;
+        const float beta = __fmul_rn(dot_fma(r.d, s2), inv_div);
+        if (beta < 0 || (FUSED_EDGE ? __fmaf_rn(da, inv_div, beta) : __fadd_rn(alpha, beta)) > 1) return false;
         const float t = __fmul_rn(dot_fma(C_A, s2), inv_div);
         if (!(r.tmin <= t && t <= tmax)) return false;
         *t_out = t;
@@ -377,7 +383,7 @@ struct TraceCount {
 // The traversal stack is the caller's local array (kStackSize entries, the
 // deeper ones past a shared-memory ring with ATRC_STACK_RING), kept out of
 // the struct so that the scalar state stays in registers.
-template <int ISECT, bool ANY, bool COUNT = false, bool EARLY = true>
+template <int ISECT, bool ANY, bool COUNT = false, bool EARLY = true, bool FUSED_EDGE = false>
 struct Tracer {
 #if ATRC_STACK_RING > 0
     int32_t* ring;
@@ -487,7 +493,7 @@ struct Tracer {
                 const float4* bc = reinterpret_cast<const float4*>(S.tri_bc) + size_t(ti) * 2;
                 hit = wt_test<ANY>(r, w, __ldg(tp), __ldg(bc), __ldg(bc + 1), best_t, &t, &u, &v);
             } else {
-                hit = mt_test<ISECT == ISECT_EXACT, ANY>(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, &t, &u, &v);
+                hit = mt_test<ISECT == ISECT_EXACT, ANY, FUSED_EDGE>(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, &t, &u, &v);
             }
             if (hit) {
                 if (ANY) { best_e = cur_entity; best_t = t; found = true; return kDone; }
@@ -590,13 +596,13 @@ struct Tracer {
     }
 };
 
-// Trace one ray to the end.  Returns true if something was hit (ANY:
-// occluded); `watchdog` is set when the traversal stack would overflow.
+// Trace one ray to the end.  Returns true if something was hit (ANY: an
+// occlusion ray of a render, occluded); `watchdog` is set when the traversal stack would overflow.
 template <int ISECT, bool ANY, bool COUNT = false>
 __device__ bool trace_ray(const Scene& S, Vec3 wo, Vec3 wd, float tmin, float tmax, Hit* hit, int* watchdog,
                           TraceCount* cnt = nullptr) {
     int32_t stack[kStackSize];
-    Tracer<ISECT, ANY, COUNT> t;
+    Tracer<ISECT, ANY, COUNT, true, ANY> t;
     t.init(S, stack, wo, wd, tmin, tmax);
     while (!t.step(S, watchdog, cnt)) {
     }
@@ -651,7 +657,7 @@ __device__ bool trace_entity(const Scene& S, int32_t ei, Vec3 wo, Vec3 wd, float
             const int32_t ti = first + k;
             const float4* tp = reinterpret_cast<const float4*>(S.tris) + size_t(ti) * 3;
             float t, u, v;
-            if (mt_test<EXACT, false>(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, &t, &u, &v)) {
+            if (mt_test<EXACT, false, false>(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, &t, &u, &v)) {
                 if (t < best_t || (t == best_t && ti < best_tri)) {
                     best_t = t; best_tri = ti; best_u = u; best_v = v;
                     r.tmax = t;
