@@ -136,7 +136,12 @@ struct Scene {
     const uint32_t* tri_orig;       // original index per pool triangle
     const Entity* entities;
     const uint32_t* tlas_order;     // TLAS leaf slot -> entity index
-    int32_t tlas_root;
+    // Top-level trees: tlas_root over boxes shrunk to the instances' vertices,
+    // for rays from within +-tlas_near on every axis (the shrunk boxes' margin
+    // covers the rounding of their transforms), tlas_far over the boxes of the
+    // instances' corners for the others (the same tree if none was shrunk).
+    int32_t tlas_root, tlas_far;
+    float tlas_near;
     int32_t entity_count;
     const Material* materials;
     const DisneyParams* disney;     // per material: its parameters if it is Disney without textures

@@ -414,7 +414,8 @@ struct Tracer {
         tmin0 = tmin;
         best_t = tmax; best_u = 0; best_v = 0;
         best_e = -1; best_tri = -1; cur_entity = -1;
-        link = S.entity_count == 0 ? kDone : S.tlas_root;
+        const bool near = max3(fabsf(o.x), fabsf(o.y), fabsf(o.z)) <= S.tlas_near;
+        link = S.entity_count == 0 ? kDone : near ? S.tlas_root : S.tlas_far;
         held = 0;
         steps = 0;
         overflow = false;

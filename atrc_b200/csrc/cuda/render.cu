@@ -338,9 +338,10 @@ constexpr int kShadowKeys = 4096;  // 16 x 16 x 16 origin cells
 // corners of its mesh's box (transform_wrapper.cpp:13-27): a rotated sphere's
 // is up to 1.7 times as wide as the sphere, and rays that only cross the
 // corners enter its tree for nothing.  With the scene, k_instance_bounds takes
-// the transformed vertices instead, and k_refit_tlas shrinks the top-level
-// boxes to them; the bounds are widened by far more than the transforms round,
-// so hits do not change (scene bound and environment keep the corner boxes).
+// the transformed vertices instead, and k_refit_tlas shrinks a copy of the
+// top-level tree to them, widened by what the transform of a ray may round
+// (HostScene::shrink_margin), so hits do not change (scene bound, environment
+// and rays from far outside the scene keep the corner boxes).
 // 64 instances: 4M incoherent queries 1.76 -> 1.58 ms, the instanced frame
 // 30.6 -> 29.0, ao 3.50 -> 3.36.
 __device__ __forceinline__ uint32_t order_bits(float x) {  // unsigned order = float order
@@ -394,7 +395,7 @@ __device__ __forceinline__ float* box_hi(Bvh4Node* n, int axis) { return reinter
 // its interior children's boxes from their nodes (boxes only shrink, and after
 // as many rounds as the tree has levels none changes).
 __global__ void __launch_bounds__(256) k_refit_tlas(Scene S, Bvh4Node* nodes, int first, int count, int depth,
-                                                   const uint32_t* bounds) {
+                                                   const uint32_t* bounds, const float* margin) {
     for (int i = threadIdx.x; i < count; i += blockDim.x) {
         Bvh4Node* n = nodes + first + i;
         for (int k = 0; k < 4; ++k) {
@@ -407,7 +408,8 @@ __global__ void __launch_bounds__(256) k_refit_tlas(Scene S, Bvh4Node* nodes, in
             for (int a = 0; a < 3; ++a) {
                 const float lo = from_order_bits(bounds[6 * ei + a]), hi = from_order_bits(bounds[6 * ei + 3 + a]);
                 if (!(lo <= hi)) continue;  // no finite vertex
-                const float pad = 1e-5f * fmaxf(fabsf(lo), fabsf(hi)) + 1e-4f * (hi - lo);
+                const float pad = margin[3 * ei + a];
+                if (!(pad < INFINITY)) continue;
                 float *bl = box_lo(n, a) + k, *bh = box_hi(n, a) + k;
                 *bl = fmaxf(*bl, lo - pad);
                 *bh = fminf(*bh, hi + pad);
@@ -437,10 +439,6 @@ __global__ void __launch_bounds__(256) k_refit_tlas(Scene S, Bvh4Node* nodes, in
         }
     }
 }
-
-// Triangles over all instances up to which their bounds are taken (48 bytes
-// each, once per scene: 2^28 are about 3 ms).
-constexpr size_t kTightTriangles = size_t(1) << 28;
 
 // Disney parameters of the constant Disney materials, once per scene.
 __global__ void k_disney_params(const Material* materials, int n, DisneyParams* out) {
@@ -2364,21 +2362,20 @@ int atrc_cuda_scene_create(const AtrcSceneDesc* desc, AtrcScene** out) {
         S.env.alias_prob = upload(d.env_alias_prob, hs->env_alias_prob, s);
         S.env.alias_idx = upload(d.env_alias_idx, hs->env_alias_idx, s);
         S.eps = 3e-4f;
-        size_t instanced = 0;
-        for (const Entity& e : hs->entities) instanced += e.flags & ENT_WRAP ? size_t(e.tri_count) : 0;
-        DevBuf bounds;
-        if (instanced > 0 && instanced <= kTightTriangles && S.tlas_root >= 0) {
+        if (!hs->shrink_margin.empty()) {
             const size_t ne = hs->entities.size();
             std::vector<uint32_t> start(6 * ne, 0u);
             for (size_t k = 0; k < ne; ++k)
                 for (int a = 0; a < 3; ++a) start[6 * k + a] = ~0u;
+            DevBuf bounds, margin;
             uint32_t* db = const_cast<uint32_t*>(upload(bounds, start, s));
+            const float* dm = upload(margin, hs->shrink_margin, s);
             const int blocks = std::max(1, int(d.sm_count * 8 / std::min<size_t>(ne, 1024)));
             k_instance_bounds<<<dim3(blocks, unsigned(std::min<size_t>(ne, 65535))), 256, 0, s>>>(S, db);
-            k_refit_tlas<<<1, 256, 0, s>>>(S, d.nodes.as<Bvh4Node>(), int(hs->tlas_first),
-                                           int(hs->nodes.size() - hs->tlas_first), hs->tlas_depth + 1, db);
+            k_refit_tlas<<<1, 256, 0, s>>>(S, d.nodes.as<Bvh4Node>(), int(hs->tlas_first + hs->tlas_count),
+                                           int(hs->tlas_count), hs->tlas_depth + 1, db, dm);
             CK(cudaGetLastError());
-            CK(cudaStreamSynchronize(s));  // `start` and `bounds` end with this scope
+            CK(cudaStreamSynchronize(s));  // the buffers end with this scope
         }
         d.scene = S;
         d.choose_default_sort(hs->entities, hs->materials);

@@ -154,6 +154,72 @@ struct HostTex {
 
 float lum(Vec3 c) { return 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z; }
 
+// Triangles over all instances up to which their top-level boxes are shrunk
+// (k_instance_bounds reads 48 bytes each, once per scene: 2^28 are about 3 ms).
+constexpr size_t kTightTriangles = size_t(1) << 28;
+
+// Sets up the top-level tree that the device shrinks to the instances'
+// vertices: a copy of the tree, the range of ray origins that may use it and
+// the margin that each shrunk box needs.
+//
+// A ray is tested in the entity's space, where its origin and direction come
+// out of 32-bit products, so a hit may lie beside the transformed triangle.
+// The displacement along local axis b is at most a few ulp of every term,
+//   e_b = kUlps u (sum_c |inv_bc| (2 O + W) + |inv_b3| + V_b) + r_b
+// (O: largest origin coordinate, 2 O + W: origin plus distance to a hit in the
+// scene's extent W, V: the mesh's reach, r: what inv(m(v)) misses v by because
+// both matrices are rounded), and along world axis a
+//   margin_a = sum_b |m_ab| e_b + kUlps u (sum_b |m_ab| V_b + |m_a3|).
+// The corner boxes kept such hits wherever the rotation made them wider than
+// the mesh; with the margin the shrunk ones do.  A box never grows: where the
+// margin exceeds the corners, they stay.  Origins beyond O (a camera far
+// outside the scene) take the corner boxes.  kReach of 16 scene extents keeps
+// the margin at 1e-4 of the extent for a rotation.
+void shrink_tlas(HostScene* hs, const std::vector<Vec3>& reach, const Bound& world) {
+    size_t instanced = 0;
+    for (const dev::Entity& e : hs->entities) instanced += e.flags & dev::ENT_WRAP ? size_t(e.tri_count) : 0;
+    if (instanced == 0 || instanced > kTightTriangles || hs->scene.tlas_root < 0) return;
+    if (hs->nodes.size() + hs->tlas_count >= size_t(INT32_MAX)) return;
+    constexpr double kReach = 16, kUlps = 16, u = 1.0 / (1 << 24);
+    double W = 0;
+    for (int k = 0; k < 3; ++k) W = std::max({W, std::fabs(double(world.lo[k])), std::fabs(double(world.hi[k]))});
+    if (!std::isfinite(W)) return;
+    const double far = 2 * kReach * W + W;
+    hs->shrink_margin.assign(3 * hs->entities.size(), INFINITY);
+    for (size_t ei = 0; ei < hs->entities.size(); ++ei) {
+        const dev::Entity& e = hs->entities[ei];
+        if (!(e.flags & dev::ENT_WRAP)) continue;
+        const float *m = e.wrap_m, *inv = e.wrap_inv;
+        const Vec3 V = reach[ei];
+        double local[3];
+        for (int b = 0; b < 3; ++b) {
+            double size = std::fabs(double(inv[4 * b + 3])) + V[b], miss = 0, shift = inv[4 * b + 3];
+            for (int c = 0; c < 3; ++c) {
+                size += std::fabs(double(inv[4 * b + c])) * far;
+                shift += double(inv[4 * b + c]) * m[4 * c + 3];
+                double p = b == c ? -1.0 : 0.0;
+                for (int k = 0; k < 3; ++k) p += double(inv[4 * b + k]) * m[4 * k + c];
+                miss += std::fabs(p) * V[c];
+            }
+            local[b] = kUlps * u * size + miss + std::fabs(shift);
+        }
+        for (int a = 0; a < 3; ++a) {
+            double margin = kUlps * u * std::fabs(double(m[4 * a + 3]));
+            for (int b = 0; b < 3; ++b) margin += std::fabs(double(m[4 * a + b])) * (local[b] + kUlps * u * V[b]);
+            hs->shrink_margin[3 * ei + a] = std::isfinite(margin) ? float(margin) : INFINITY;
+        }
+    }
+    const int32_t shift = int32_t(hs->tlas_count);
+    for (size_t k = 0; k < hs->tlas_count; ++k) {
+        Bvh4Node n = hs->nodes[hs->tlas_first + k];
+        for (int32_t& l : n.link)
+            if (l >= 0) l += shift;
+        hs->nodes.push_back(n);
+    }
+    hs->scene.tlas_root += shift;
+    hs->scene.tlas_near = float(kReach * W);
+}
+
 }  // namespace
 
 void build_host_scene(const AtrcSceneDesc& d, HostScene* hs, int device) {
@@ -336,6 +402,7 @@ void build_host_scene(const AtrcSceneDesc& d, HostScene* hs, int device) {
     // ------------------------------------------------------------ entities
     std::vector<bool> leaf_needs_alias(d.geometry_count, false);
     std::vector<Bound> ent_bounds(d.entity_count);
+    std::vector<Vec3> leaf_reach(d.entity_count);  // largest |coordinate| of the leaf's vertices
     for (uint32_t ei = 0; ei < d.entity_count; ++ei) {
         const AtrcEntityDesc& e = d.entities[ei];
         if (e.geometry < 0 || uint32_t(e.geometry) >= d.geometry_count) throw std::runtime_error("bad geometry index");
@@ -386,6 +453,7 @@ void build_host_scene(const AtrcSceneDesc& d, HostScene* hs, int device) {
             b = L.bound;
         }
         ent_bounds[ei] = b;
+        for (int k = 0; k < 3; ++k) leaf_reach[ei][k] = std::max(std::fabs(L.bound.lo[k]), std::fabs(L.bound.hi[k]));
     }
     // triangle-area alias tables for mesh lights
     std::vector<int32_t> leaf_alias(d.geometry_count, -1);
@@ -414,14 +482,18 @@ void build_host_scene(const AtrcSceneDesc& d, HostScene* hs, int device) {
         hs->tlas_depth = tl.max_depth;
         hs->tlas_first = hs->nodes.size();
         hs->scene.tlas_root = collapse_bvh4(tl, &hs->nodes);
+        hs->tlas_count = hs->nodes.size() - hs->tlas_first;
         validate_bvh4(hs->nodes, hs->scene.tlas_root, 0, uint32_t(d.entity_count));
         hs->tlas_order = tl.order;
     } else {
         hs->scene.tlas_root = 0;
     }
+    hs->scene.tlas_far = hs->scene.tlas_root;
+    hs->scene.tlas_near = 0;
     hs->scene.entity_count = int32_t(d.entity_count);
     Bound world;
     for (auto& b : ent_bounds) world.add(b);
+    shrink_tlas(hs, leaf_reach, world);
     for (int k = 0; k < 3; ++k) { hs->scene.scene_lo[k] = world.lo[k]; hs->scene.scene_hi[k] = world.hi[k]; }
 
     // ------------------------------------------------------------ textures

@@ -13,7 +13,7 @@
 namespace atrc {
 
 struct HostScene {
-    std::vector<Bvh4Node> nodes;  // every 4-wide node (each BLAS, then the TLAS)
+    std::vector<Bvh4Node> nodes;  // every 4-wide node (each BLAS, then the TLAS, then its copy)
     std::vector<float> tris;          // 12 per triangle
     std::vector<float> tri_bc;        // 8 per triangle: exact B and C
     std::vector<dev::TriShade> tri_shade;
@@ -31,7 +31,13 @@ struct HostScene {
     std::vector<int32_t> env_alias_idx;
     dev::Scene scene{};               // pointers left null; filled on upload
     int max_blas_depth = 0, tlas_depth = 0;
-    size_t tlas_first = 0;  // the top-level tree's nodes are nodes[tlas_first ...]
+    // The top-level tree over the instances' corner boxes is nodes[tlas_first,
+    // tlas_first + tlas_count), scene.tlas_far; a second copy behind it
+    // (scene.tlas_root), where there is one, is shrunk on the device to the
+    // instances' vertices, widened by shrink_margin (xyz per entity, world
+    // space; infinite for an entity that keeps its corner box).
+    size_t tlas_first = 0, tlas_count = 0;
+    std::vector<float> shrink_margin;
 };
 
 // Throws std::runtime_error with a message on unsupported or invalid input.
