@@ -473,11 +473,12 @@ constexpr int kIssuePools = 4;
 
 // Counters for the next iteration: what the last one did, how many samples
 // the next may issue, and whether the work is done.  Runs on one thread, at
-// the end of k_init and of k_finish's last block.
-__device__ void begin_iteration(Counters* c, int cap) {
-    if (c->iterations > 0)
+// the end of k_init (nothing was done yet) and of k_finish's last block.
+__device__ void begin_iteration(Counters* c, int cap, bool first) {
+    if (!first) {
         for (int k = 0; k < 3; ++k) c->stage_ns[k] += c->mark[k + 1] - c->mark[k];
-    c->iterations++;
+        c->iterations++;
+    }
     c->rays_shadow += c->n_shadow;
     // what the last iteration issued, and the slots it took and freed
     const int issued = min(c->gen_ticket, c->n_new);
@@ -522,7 +523,7 @@ __global__ void k_init(Pool P, int cap, int nkeys, Counters* c, unsigned long lo
         c->total = total;
         c->out = 0;
         c->t_start = global_ns();
-        begin_iteration(c, cap);
+        begin_iteration(c, cap, true);
     }
 }
 
@@ -1861,7 +1862,7 @@ __global__ void k_finish(Params p, Pool P, Counters* c) {
         if (atomicAdd(&c->finished_blocks, 1) == int(gridDim.x) - 1) {
             __threadfence();
             c->finished_blocks = 0;
-            begin_iteration(c, P.cap);
+            begin_iteration(c, P.cap, false);
         }
     }
 }
