@@ -470,6 +470,13 @@ __global__ void k_loop_cond(Counters* c, cudaGraphConditionalHandle h, int max_w
 // much sky takes several pools of samples per iteration.  The bound keeps the
 // host's progress and cancel polls (one per window of iterations) frequent.
 constexpr int kIssuePools = 4;
+constexpr int kMinLanes = 16;  // k_extend: reserved slots with which a warp goes on without a full 32
+// Bounds of an iteration's counters, which are ints.  A warp of k_extend asks
+// for 32 slots whenever it holds fewer, for each kMinLanes samples it takes at
+// the least, so slot_ticket may run to 32 / kMinLanes times the samples issued
+// beyond the slots there are (and 32 for each of at most 2^18 warps).
+constexpr unsigned long long kMaxPool = 1ull << 28, kMaxIssue = 1ull << 29;
+static_assert(32 / kMinLanes * kMaxIssue + kMaxPool + (32ull << 18) < (1ull << 31), "slot_ticket and gen_ticket fit an int");
 
 // Counters for the next iteration: what the last one did, how many samples
 // the next may issue, and whether the work is done.  Runs on one thread, at
@@ -490,7 +497,7 @@ __device__ void begin_iteration(Counters* c, int cap, bool first) {
     c->in = c->out;
     c->out = c->in ^ 1;
     const unsigned long long remaining = c->total - c->issued;
-    const unsigned long long most = c->n_free > 0 ? (unsigned long long)kIssuePools * cap : 0;
+    const unsigned long long most = c->n_free > 0 ? min((unsigned long long)kIssuePools * cap, kMaxIssue) : 0;
     c->n_new = int(remaining < most ? remaining : most);
     c->gen_base = c->issued;
     c->gen_ticket = 0;
@@ -1009,7 +1016,6 @@ __device__ __forceinline__ void retire_path(const Scene& S, const Params& p, Poo
 // 36.2 -> 33.3 ms, media 29.0 -> 25.9, subsurface Cornell 6.61 -> 6.36).
 template <int ISECT, bool COUNT, bool CONT>
 __global__ void __launch_bounds__(kTraceBlock, ATRC_TRACE_MIN_BLOCKS) k_extend(Scene S, Params p, Pool P, Counters* c) {
-    constexpr int kMinLanes = 16;  // reserved slots a warp goes on with
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     if (CONT) mark_stage(c, 0);
@@ -2642,7 +2648,7 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
     const int nl = shadow_rays_per_path(d.scene, *desc);
     size_t cap = desc->path_pool > 0 ? size_t(desc->path_pool) : size_t(d.tuned_pool);
     cap = std::min<size_t>(cap, std::max<unsigned long long>(total, 1024ULL));
-    cap = std::min<size_t>(cap, (size_t(1) << 28) / nl);
+    cap = std::min<size_t>(cap, kMaxPool / nl);
     const size_t shadow_cap = cap * nl;
     const PoolLayout L = pool_layout(cap, shadow_cap, p.nkeys);
     // the buffer only grows: a smaller pool is laid out inside it (k_init
