@@ -939,10 +939,9 @@ int atrc_guide_pdf(AtrcGuide* g, const float* queries, const float* dirs, size_t
 // One Adam step on `n` records at `records` (device) -- internal helper.
 static void train_step(GuideImpl& G, const GuideRecord* rec, int n, float* loss_out) {
     cudaStream_t s = G.stream;
-    float* sc = G.scratch.as<float>();  // [1] loss, [4] live records, [8, 9] target sum in 64 bits
-    double* wsum = reinterpret_cast<double*>(sc + 8);
-    CK(cudaMemsetAsync(sc + 1, 0, sizeof(float), s));
-    CK(cudaMemsetAsync(wsum, 0, sizeof(double), s));
+    float* sc = G.scratch.as<float>();  // [0, 1] target sum in 64 bits, [2] loss, [4] live records
+    double* wsum = G.scratch.as<double>();
+    CK(cudaMemsetAsync(sc, 0, 3 * sizeof(float), s));
     k_target_sum<<<G.sm_count * 2, 256, 0, s>>>(rec, n, wsum);
     TrainArgs a;
     a.rec = rec;
@@ -950,7 +949,7 @@ static void train_step(GuideImpl& G, const GuideRecord* rec, int n, float* loss_
     a.weight_sum = wsum;
     a.grad_w = G.w_g.as<float>();
     a.grad_table = G.t_g.as<float>();
-    a.loss = sc + 1;
+    a.loss = sc + 2;
     a.target_clamp = G.desc.target_clamp;
     const int tiles = (n + kTile - 1) / kTile;
     k_guide_train<<<std::min(tiles, G.sm_count), kTile, kTrSmem, s>>>(G.view(), a, G.err.as<int>());
@@ -967,7 +966,7 @@ static void train_step(GuideImpl& G, const GuideRecord* rec, int n, float* loss_
     k_guide_adam<__half><<<G.sm_count * 8, 256, 0, s>>>(G.t_f.as<float>(), G.t_g.as<float>(), G.t_m.as<float>(),
                                                         G.t_v.as<float>(), G.t_h.as<__half>(), G.table_n, ad);
     CK(cudaGetLastError());
-    if (loss_out) CK(cudaMemcpyAsync(loss_out, sc + 1, sizeof(float), cudaMemcpyDeviceToHost, s));
+    if (loss_out) CK(cudaMemcpyAsync(loss_out, sc + 2, sizeof(float), cudaMemcpyDeviceToHost, s));
 }
 
 int atrc_guide_train(AtrcGuide* g, int steps, float* last_loss) {
@@ -1049,9 +1048,8 @@ int atrc_guide_gradients(AtrcGuide* g, const float* records, size_t n, float* gr
         cudaStream_t s = G.stream;
         CK(cudaMemcpyAsync(G.records.p, records, n * sizeof(GuideRecord), cudaMemcpyHostToDevice, s));
         float* sc = G.scratch.as<float>();
-        double* wsum = reinterpret_cast<double*>(sc + 8);
-        CK(cudaMemsetAsync(sc + 1, 0, sizeof(float), s));
-        CK(cudaMemsetAsync(wsum, 0, sizeof(double), s));
+        double* wsum = G.scratch.as<double>();
+        CK(cudaMemsetAsync(sc, 0, 3 * sizeof(float), s));
         CK(cudaMemsetAsync(G.w_g.p, 0, kWeights * sizeof(float), s));
         CK(cudaMemsetAsync(G.t_g.p, 0, G.table_n * sizeof(float), s));
         const GuideRecord* rec = G.records.as<GuideRecord>();
@@ -1062,7 +1060,7 @@ int atrc_guide_gradients(AtrcGuide* g, const float* records, size_t n, float* gr
         a.weight_sum = wsum;
         a.grad_w = G.w_g.as<float>();
         a.grad_table = G.t_g.as<float>();
-        a.loss = sc + 1;
+        a.loss = sc + 2;
         a.target_clamp = G.desc.target_clamp;
         const int tiles = int((n + kTile - 1) / kTile);
         k_guide_train<<<std::min(tiles, G.sm_count), kTile, kTrSmem, s>>>(G.view(), a, G.err.as<int>());
@@ -1070,7 +1068,7 @@ int atrc_guide_gradients(AtrcGuide* g, const float* records, size_t n, float* gr
         CK(cudaMemcpyAsync(grad_weights, G.w_g.p, kWeights * sizeof(float), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(grad_table, G.t_g.p, G.table_n * sizeof(float), cudaMemcpyDeviceToHost, s));
         float l = 0;
-        CK(cudaMemcpyAsync(&l, sc + 1, sizeof(float), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(&l, sc + 2, sizeof(float), cudaMemcpyDeviceToHost, s));
         CK(cudaMemsetAsync(G.w_g.p, 0, kWeights * sizeof(float), s));
         CK(cudaMemsetAsync(G.t_g.p, 0, G.table_n * sizeof(float), s));
         check_err(G, "atrc_guide_gradients");
