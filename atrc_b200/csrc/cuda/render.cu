@@ -1749,12 +1749,12 @@ __device__ __forceinline__ void shadow_ray(const Scene& S, Pool& P, Counters* c,
 
 // Occlusion rays.  WARPS: the warps that fit the GPU take 32 rays at a time,
 // their first by their place in the grid and the next from a cursor, so that no
-// block waits for its slowest warp; else one ray per thread of a grid that
-// covers the queue.  In large scenes, whose rays differ most in length, the
-// warps win (with 48 registers, occlusion rays of the room 10.1 -> 9.7 ms, of
-// ao on the instanced scene 2.15 -> 2.02, of the guided room 3.08 -> 2.91), in
-// small ones the blocks (Cornell 1.68 against 1.78, media 0.76 against 1.02):
-// kShadowWarps.
+// block waits for its slowest warp and a short queue starts no empty blocks;
+// else one ray per thread of a grid that covers the queue, without the cursor's
+// traffic on one address, which shows where a ray takes few steps
+// (choose_shadow_schedule).  Occlusion rays of a render, blocks -> warps: room
+// 1280x720 4.41 -> 4.13 ms, ao of the instanced scene 0.95 -> 0.91 and at
+// 640x360 0.223 -> 0.207; Cornell 0.468 -> 0.506, media 767x511 0.52 -> 0.61.
 template <int ISECT, bool COUNT, bool WARPS>
 __global__ void __launch_bounds__(kTraceBlock, ATRC_SHADOW_MIN_BLOCKS) k_shadow(Scene S, Pool P, Counters* c) {
     if (!P.shadow_sort) mark_stage(c, 2);
@@ -1767,6 +1767,7 @@ __global__ void __launch_bounds__(kTraceBlock, ATRC_SHADOW_MIN_BLOCKS) k_shadow(
         while (base < n) {
             if (base + lane < n) shadow_ray<ISECT, COUNT>(S, P, c, base + lane, &tc);
             __syncwarp();
+            if (n <= all) break;  // the grid held every ray
             if (lane == 0) base = all + atomicAdd(&c->sh_cursor, 32);
             base = __shfl_sync(0xffffffffu, base, 0);
         }
@@ -2002,7 +2003,7 @@ struct DeviceSceneImpl {
     int tuned_shadow_fetch = 0;   // k_shadow_fetch instead of k_shadow
     int tuned_shadow_sort = 0;    // shadow queue in origin-cell order
     int default_sort = ATRC_SORT_NONE;  // tuned_sort until the scene is tuned
-    bool shadow_warps = false;          // k_shadow by warps (kShadowWarps triangles and more)
+    bool shadow_warps = false;          // k_shadow by warps (choose_shadow_schedule)
     int tuned_trials = 0;
     double tuned_ms = 0, default_ms = 0;
     DevBuf tune_film;
@@ -2026,6 +2027,19 @@ struct DeviceSceneImpl {
         }
         default_sort = scene.has_media || (disney && other) ? ATRC_SORT_TYPE : ATRC_SORT_NONE;
         tuned_sort = default_sort;
+    }
+    // Occlusion rays by warps, except where they take few steps: in scenes with
+    // media, whose vertices lie in empty space (the media scene with 180 to
+    // 512,000 triangles: warps take 1.17 to 1.20 times as long, a render 1 %
+    // longer), and in scenes of a few primitives (16: 1.6 times, 36: 1.04 to
+    // 1.08, the render 1 %).  In all others, from 8 instances of meshes of 8 and
+    // 20 triangles to rooms of 997,600 triangles and 64 instances of 3.1M,
+    // warps take 0.75 to 1.0 times as long at 1280x720 and 640x360.
+    void choose_shadow_schedule(const std::vector<Entity>& entities) {
+        constexpr size_t kFewPrimitives = 64;
+        size_t primitives = 0;
+        for (const Entity& e : entities) primitives += size_t(std::max(e.tri_count, 1));
+        shadow_warps = !scene.has_media && primitives >= kFewPrimitives;
     }
     void ensure_render_resources() {
         if (!ev0) {
@@ -2111,11 +2125,6 @@ int shadow_grid(size_t shadow_cap, int sm_count, bool warps) {
     const size_t full = (shadow_cap + 127) / 128;
     return int(std::min<size_t>(full, size_t(sm_count) * ATRC_SHADOW_MIN_BLOCKS * (warps ? 1 : kShadowGridWaves)));
 }
-// Triangles from which the occlusion rays go by warps: between the largest
-// scene measured for blocks (media, 200,040) and the smallest for warps (room,
-// 403,000).
-constexpr size_t kShadowWarps = size_t(1) << 18;
-
 PoolLayout pool_layout(size_t cap, size_t shadow_cap, int nkeys) {
     PoolLayout L{};
     size_t o = 0;
@@ -2386,7 +2395,7 @@ int atrc_cuda_scene_create(const AtrcSceneDesc* desc, AtrcScene** out) {
         }
         d.scene = S;
         d.choose_default_sort(hs->entities, hs->materials);
-        d.shadow_warps = hs->tri_orig.size() >= kShadowWarps;
+        d.choose_shadow_schedule(hs->entities);
         d.watchdog.alloc(2 * sizeof(int));  // [0] watchdog code, [1] ray-query cursor
         // load the module's static scratch onto this device now, so that
         // atrc_cuda_render_noalloc neither allocates nor looks it up itself
