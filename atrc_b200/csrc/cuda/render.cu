@@ -2002,22 +2002,34 @@ struct DeviceSceneImpl {
     int tuned_queue = 0;          // extend queue in slot order (1) or shade order (0)
     int tuned_shadow_fetch = 0;   // k_shadow_fetch instead of k_shadow
     int tuned_shadow_sort = 0;    // shadow queue in origin-cell order
-    int default_sort = ATRC_SORT_NONE;  // tuned_sort until the scene is tuned
+    int default_sort = ATRC_SORT_NONE;  // tuned_sort until the scene is tuned,
+    bool sort_tuned = false;            // in renders of kSortSamples and more
     bool shadow_warps = false;          // k_shadow by warps (choose_shadow_schedule)
     int tuned_trials = 0;
     double tuned_ms = 0, default_ms = 0;
     DevBuf tune_film;
-    void resolve_sort(Params* p, int requested) const {
-        p->sort_mode = requested == ATRC_SORT_AUTO ? tuned_sort : requested;
+    void resolve_sort(Params* p, int requested, unsigned long long samples) const {
+        p->sort_mode = requested != ATRC_SORT_AUTO ? requested
+                       : sort_tuned || samples >= kSortSamples ? tuned_sort : int(ATRC_SORT_NONE);
         p->slot_queue = tuned_queue;
         p->nkeys = std::max(scene.material_count, kMaterialTypes) + 2;
     }
     // The sort of a scene that was not tuned: by material type where shading
     // differs most between neighbouring paths, media (tracking loops against
-    // surfaces; 767x511x8: 24.4 -> 22.9 ms) and Disney among other materials
-    // (subsurface Cornell 6.01 -> 5.01).  Where all is Disney the sort only
-    // costs (room 49.5 -> 50.5), and a box of Lambertian walls gains nothing
-    // (10.6 -> 10.8): black surfaces end their paths and do not count.
+    // surfaces; 767x511x8: 24.8 -> 23.1 ms) and Disney among other materials
+    // (subsurface Cornell 512x512x16 12.9 -> 10.3, Cornell with half or one of
+    // its walls Disney 9.9 -> 9.4 and 10.0 -> 9.4, seven materials with media
+    // 6.9 -> 4.3, a room with every fourth or one material Lambertian 22.1 ->
+    // 21.4 and 21.1 -> 20.6).  Where most rays end in the sky there is little to
+    // shade, and the mixed scene pays for the sort (64 instances with one, eight
+    // or 32 of them Lambertian 5.42 -> 5.51, 5.61 -> 5.70, 5.94 -> 5.99).  Where
+    // all is Disney it only costs (room 20.8 -> 21.0), and a box of Lambertian
+    // walls gains nothing (8.9 -> 9.1): black surfaces end their paths and do not
+    // count.  The sort is two launches per iteration: below kSortSamples they
+    // cost more than they give (at 2^12 to 2^17 samples all of these scenes are
+    // slower with it, by 2 to 7 %; 2^18 is even; at 2^19 they are 1 to 9 %
+    // faster, the instances 1 % slower).
+    static constexpr unsigned long long kSortSamples = 1ull << 19;
     void choose_default_sort(const std::vector<Entity>& entities, const std::vector<Material>& materials) {
         bool disney = false, other = false;
         for (const Entity& e : entities) {
@@ -2629,7 +2641,6 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
     d.scene.eps = desc->eps;
     d.scene.disney_fixed = desc->disney_fixed;
     Params p = make_params(*desc);
-    d.resolve_sort(&p, desc->sort_mode);
     // views, their tile tables and sample ranges
     std::vector<View> views(nviews);
     size_t table_bytes = 0;
@@ -2652,6 +2663,7 @@ static int render_impl(AtrcScene* scene, const AtrcRenderDesc* descs, const Atrc
             tb += (tile_table_bytes(views[v]) + 255) & ~size_t(255);
         }
     }
+    d.resolve_sort(&p, desc->sort_mode, total);
     // path pool: enough paths to fill the GPU; shadow capacity = pool x
     // shadow rays one path can emit in one iteration
     const int nl = shadow_rays_per_path(d.scene, *desc);
@@ -3045,6 +3057,7 @@ int atrc_cuda_set_tuning(AtrcScene* scene, const AtrcTuning* in) {
     DeviceSceneImpl& d = scene->impl;
     d.tuned_pool = in->path_pool;
     d.tuned_sort = in->sort_mode;
+    d.sort_tuned = true;
     d.tuned_gen_blocks = in->gen_blocks_per_sm;
     d.tuned_gen_threads = in->gen_threads;
     d.tuned_fin_threads = in->finish_threads;
@@ -3234,12 +3247,12 @@ int atrc_cuda_render_noalloc(AtrcScene* scene, const AtrcRenderDesc* desc, const
         d.scene.eps = desc->eps;
         d.scene.disney_fixed = desc->disney_fixed;
         Params p = make_params(*desc);
-        d.resolve_sort(&p, desc->sort_mode);
         View view = make_view(*desc);
         const int spp = desc->spp_count > 0 ? desc->spp_count : desc->spp;
         view.start = 0;
         view.count = (unsigned long long)view.SW * view.SH * spp;
         const unsigned long long total = view.count;
+        d.resolve_sort(&p, desc->sort_mode, total);
         // the path state packs (view << kTileBits) | tile: a larger tile grid
         // would spill into the view bits
         if (size_t(view.TX) * view.TY >= (size_t(1) << kTileBits))

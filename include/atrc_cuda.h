@@ -321,9 +321,10 @@ typedef enum AtrcRendererType {
 
 /* Sorting of hit records before shading (a counting sort by key). */
 typedef enum AtrcSortMode {
-    ATRC_SORT_AUTO     = -1,  /* the scene's tuned choice; untuned, TYPE with  */
-                              /* media or with Disney among other materials,   */
-                              /* else NONE                                     */
+    ATRC_SORT_AUTO     = -1,  /* the scene's tuned choice; untuned, TYPE in    */
+                              /* renders of 2^19 samples and more of scenes    */
+                              /* with media or with Disney among other         */
+                              /* materials, else NONE                          */
     ATRC_SORT_NONE     = 0,   /* shade in extend-queue order                   */
     ATRC_SORT_TYPE     = 1,   /* by material type (miss / each type / medium)  */
     ATRC_SORT_MATERIAL = 2    /* by material index (miss / each / medium)      */

@@ -90,3 +90,23 @@ def test_kept_graphs_follow_the_call(tmp_path):
         fresh = DeviceScene(cfg)
         own = Guide.for_scene(fresh, log2_table=12) if guided else None
         _same(got, call(fresh, own, changes, gbuffer, callback, guided, record), f"step {i}: {steps[i]}")
+
+
+@pytest.mark.parametrize("height", [255, 256])
+def test_default_sort_starts_at_its_size(tmp_path, height):
+    cfg = _feature_config(tmp_path)
+    desc, _ = cfg.rendering(0)
+    desc.width, desc.height, desc.spp, desc.task_grid_size = 512, height, 4, 4096
+    dev = DeviceScene(cfg)
+    films, launches = {}, {}
+    for mode in (-1, 0, 1):
+        desc.sort_mode = mode
+        films[mode] = Film(desc.width, desc.height)
+        st = dev.render(desc, films[mode])
+        launches[mode] = st["kernel_launches"]
+        assert st["samples"] == 512 * height * 4
+    assert launches[-1] == launches[1 if height == 256 else 0] and launches[0] < launches[1]
+    _same(films[-1], films[0], "auto")
+    dev.set_tuning(sort_mode=2)  # chosen by the caller: at every size
+    desc.sort_mode = -1
+    assert dev.render(desc, Film(desc.width, desc.height))["kernel_launches"] == launches[1]
