@@ -1946,7 +1946,7 @@ struct DeviceSceneImpl {
         alias_idx, env_probs, env_alias_prob, env_alias_idx;
     DevBuf watchdog;
     DevBuf tiles;  // tile tables of the film's sample grid
-    DevBuf ray_buf;            // rays and hits of host queries (at most kRayKeep rays)
+    DevBuf ray_buf;            // rays and hits of host queries (at most kRayKeep rays), kept with the scene
     void* ray_stage = nullptr;  // pinned: rays, hits and the watchdog word of small host queries
     size_t ray_stage_rays = 0;
     static constexpr size_t kRayKeep = size_t(1) << 20;   // 48 MB
@@ -1991,12 +1991,13 @@ struct DeviceSceneImpl {
     void* stage = nullptr;             // pinned host staging for host films
     size_t stage_bytes = 0;
     // launch configuration (atrc_cuda_autotune chooses it; these are the
-    // defaults): ATRC_SORT_AUTO resolves to tuned_sort, path_pool 0 to
-    // tuned_pool; k_generate / k_finish use the grid and block shapes
+    // defaults): ATRC_SORT_AUTO resolves to tuned_sort (resolve_sort),
+    // path_pool 0 to tuned_pool; k_free_slots / k_finish use the grid and
+    // block shapes
     int tuned_sort = ATRC_SORT_NONE;
     int tuned_pool = 1 << 21;
-    int tuned_gen_blocks = 16;    // k_generate / k_finish blocks per SM
-    int tuned_gen_threads = 256;  // k_generate block
+    int tuned_gen_blocks = 16;    // k_free_slots / k_finish blocks per SM
+    int tuned_gen_threads = 256;  // k_free_slots block
     int tuned_fin_threads = 128;  // k_finish block
     int tuned_fetch = 0;          // k_extend_fetch instead of k_extend
     int tuned_queue = 0;          // extend queue in slot order (1) or shade order (0)

@@ -201,9 +201,9 @@ def reference_arm(args, rank: int, world: int) -> None:
 # DRAM bytes per closest ray of k_extend on the instanced workload, from one
 # ncu capture of every k_extend launch of an NVTX-marked 2-spp step
 # (dram__bytes_read.sum + dram__bytes_write.sum summed over the launches,
-# divided by the step's closest rays: 1,571.9 MB / 5,305,924 rays; the kernel
+# divided by the step's closest rays: 1,571.1 MB / 5,305,924 rays; the kernel
 # makes the camera rays, writes new paths and splats the misses, too).
-K_EXTEND_DRAM_BYTES_PER_RAY = 296.2
+K_EXTEND_DRAM_BYTES_PER_RAY = 296.1
 
 
 def stream_read_peaks(device: int) -> dict:
@@ -371,9 +371,11 @@ def media_comparison(args, l2_peak: float) -> dict:
             "ms_per_step": sec / args.media_steps * 1e3,
             "rays_closest_per_sample": rays / samples, "rays_shadow_per_sample":
                 sum(st["rays_shadow"] for st in stats) / samples,
+            # stages by device timestamps: extend holds camera rays, closest
+            # hits, splats of misses and the material sort
             "kernel_time_share": {"extend": ext / sec, "shade": sum(st["shade_seconds"] for st in stats) / sec,
                                   "shadow": sum(st["shadow_seconds"] for st in stats) / sec},
-            "roofline": {"bound": "l2", "kernel": "k_extend (closest-hit traversal)", "achieved": achieved,
+            "roofline": {"bound": "l2", "kernel": "k_extend (camera rays, closest-hit traversal, splats of misses)", "achieved": achieved,
                          "peak": l2_peak, "unit": "GB/s", "frac": achieved / l2_peak, "bytes_per_ray": bpr},
             "cpu_baseline": {"value": cpu_samples / cpu_s / 1e6, "unit": "Msamples/s", "cores": cpu.threads,
                              "kind": cpu.kind, "sample": f"1 spp of one in {stride} of the 32x32 tiles ({cpu_samples} "
@@ -426,7 +428,7 @@ def batch_comparison(args) -> dict:
         guide.train(steps=4)
     q = lambda a: {"median_s": float(np.median(a)), "p90_s": float(np.quantile(a, 0.9)), "max_s": float(np.max(a))}  # noqa: E731
 
-    def compare(views, device_loop_one_by_one: bool):
+    def compare(views):
         samples = sum(v.width * v.height * v.spp for v in views)
         films = [Film(v.width, v.height, device=True) for v in views]
         dev.render_batch(views[:2], films[:2], guide=guide)       # warm-up (graph, buffers)
@@ -450,23 +452,13 @@ def batch_comparison(args) -> dict:
                "one_by_one": {"seconds": t_one, "Msamples_per_s": samples / t_one / 1e6, "completion": q(one_secs),
                               "loop": "atrc_cuda_render_guided per view"},
                "speedup": t_one / t_batch}
-        if device_loop_one_by_one:
-            # the same views one by one through the device-side loop: what
-            # sharing one path pool gains, apart from the loop itself
-            t0 = time.perf_counter()
-            for v, f in zip(views, films):
-                f.clear()
-                dev.render_batch([v], [f], guide=guide)
-            t_one_loop = time.perf_counter() - t0
-            out["one_by_one_device_loop"] = {"seconds": t_one_loop, "Msamples_per_s": samples / t_one_loop / 1e6}
-            out["speedup_vs_device_loop"] = t_one_loop / t_batch
         return out
-    full = compare(batch_views(cfg, args.batch_views, 1004, args.batch_spp_scale), True)
+    full = compare(batch_views(cfg, args.batch_views, 1004, args.batch_spp_scale))
     # the regime batching is for: many small views that cannot fill the GPU alone
     small = batch_views(cfg, args.batch_views, 1005, 1.0 / 64)
     for v in small:
         v.width = v.height = 128 if v.width < 1024 else 256
-    small_r = compare(small, False)
+    small_r = compare(small)
     return {"workload": f"indoor_room_{args.batch_views}_views", "spp_scale": args.batch_spp_scale,
             "tuning": {k: tuning[k] for k in ("path_pool", "sort_mode", "gen_blocks_per_sm", "gen_threads",
                                               "finish_threads", "extend_fetch", "queue_order", "shadow_fetch", "shadow_sort")},
@@ -607,7 +599,10 @@ def main():
     nodes_per_ray = cstats["nodes_closest"] / crays
     tris_per_ray = cstats["tris_closest"] / crays
     ents_per_ray = cstats["ents_closest"] / crays
-    bytes_per_ray = nodes_per_ray * 112 + tris_per_ray * 48 + ents_per_ray * 64 + 56
+    # a camera ray is made in registers; a continuing path's ray is read from
+    # its queue entry (4 bytes) and record (32)
+    continuing = max(rays_closest - samples / world, 0) / max(rays_closest, 1)
+    bytes_per_ray = nodes_per_ray * 112 + tris_per_ray * 48 + ents_per_ray * 64 + continuing * 36
     achieved = bytes_per_ray * rays_closest / max(ext_time, 1e-9) / 1e9
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     hbm_peak = float(peaks.get("hbm_gbs", 6650.0))
@@ -641,11 +636,11 @@ def main():
                                                          "finish_threads", "extend_fetch", "queue_order", "shadow_fetch", "shadow_sort", "trials")}},
             "e2e": {"value": e2e_value, "unit": "Msamples/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": d2h},
             # k_extend reads its nodes and triangles mostly from L1 / L2 (ncu:
-            # 235 of ~1,800 algorithmic bytes per ray come from DRAM), so its
+            # 296 of ~1,800 algorithmic bytes per ray come from DRAM), so its
             # bound is the cache hierarchy: the algorithmic bytes are reported
             # against the L2 streaming-read peak measured in this run, and its
             # DRAM traffic against the HBM copy peak beside it
-            "roofline": {"bound": "l2", "kernel": "k_extend (closest-hit traversal)", "achieved": achieved,
+            "roofline": {"bound": "l2", "kernel": "k_extend (camera rays, closest-hit traversal, splats of misses)", "achieved": achieved,
                          "peak": l2_peak, "unit": "GB/s", "frac": achieved / l2_peak,
                          "peak_source": (f"measured in this run: streaming read of an L2-resident "
                                          f"{stream['l2_buffer_mb']} MB buffer (atrc_cuda_stream_read_gbs)"),
@@ -660,6 +655,8 @@ def main():
                          "bytes_per_ray": bytes_per_ray, "nodes_per_ray": nodes_per_ray,
                          "tris_per_ray": tris_per_ray, "entities_per_ray": ents_per_ray,
                          "avg_launch_ms": avg_launch_s * 1e3},
+            # stages by device timestamps: extend holds camera rays, closest
+            # hits, splats of misses and the material sort
             "kernel_time_share": {"extend": ext_time / elapsed, "shade": shade_time / elapsed,
                                   "shadow": shadow_time / elapsed},
             "rays": {"closest_per_sample": rays_closest / max(samples / world, 1),

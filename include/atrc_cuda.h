@@ -475,7 +475,9 @@ void atrc_cuda_scene_destroy(AtrcScene* scene);
  * ANY mode writes t = 1 / entity = 0 for an occluded ray and t = -1 otherwise.
  * `exact` is an AtrcIsectMode: 1 selects the reference-exact Moller-Trumbore
  * test (same operation order, no fused multiply-add), 0 the fast test, 2 the
- * watertight test. */
+ * watertight test.  The scene keeps buffers for batches of up to 2^20 rays (48
+ * MB on the device) and a pinned stage for up to 2^17 (6 MB) from the first
+ * batch that needs them until it is destroyed. */
 int atrc_cuda_trace_rays(AtrcScene* scene, const AtrcRay* rays, size_t n,
                          AtrcHit* hits, int mode, int exact);
 
