@@ -353,7 +353,9 @@ def media_comparison(args, l2_peak: float) -> dict:
     sec = ev0.elapsed_time(ev1) / 1e3
     samples = desc.width * desc.height * spp * args.media_steps
     crays = max(cst["rays_closest"], 1)
-    bpr = (cst["nodes_closest"] * 112 + cst["tris_closest"] * 48 + cst["ents_closest"] * 64) / crays + 56
+    # a continuing path's ray is read from its queue entry and record (4 + 32 bytes)
+    bpr = (cst["nodes_closest"] * 112 + cst["tris_closest"] * 48 + cst["ents_closest"] * 64
+           + max(cst["rays_closest"] - cst["samples"], 0) * 36) / crays
     ext = sum(st["extend_seconds"] for st in stats)
     rays = sum(st["rays_closest"] for st in stats)
     achieved = bpr * rays / max(ext, 1e-9) / 1e9
